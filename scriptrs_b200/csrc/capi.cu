@@ -117,6 +117,7 @@ int32_t frontend_run(sb_ctx* c, const void* d_pcm, SampleFormat fmt, const int64
     std::vector<int64_t> meta(3 * n1);  // starts | lens | frame prefix sums
     int64_t* fo = meta.data() + 2 * n1;
     fo[0] = 0;
+    int max_frames = 0;
     for (int64_t i = 0; i < n_clips; ++i) {
         if (clip_len[i] <= 0) return fail(SB_EMPTY_AUDIO, "audio input was empty");  // frontend.rs:105
         meta[i] = clip_start[i];
@@ -124,6 +125,7 @@ int32_t frontend_run(sb_ctx* c, const void* d_pcm, SampleFormat fmt, const int64
         const int64_t t = frames_for_samples(clip_len[i]);
         if (t > INT32_MAX / 2) return fail(SB_INVALID_ARGUMENT, "clip too long");
         fo[i + 1] = fo[i] + t;
+        max_frames = std::max(max_frames, (int)t);
     }
     if (frame_offsets) std::memcpy(frame_offsets, fo, sizeof(int64_t) * n1);
     SB_CUDA(cudaSetDevice(c->device));
@@ -132,13 +134,12 @@ int32_t frontend_run(sb_ctx* c, const void* d_pcm, SampleFormat fmt, const int64
     SB_CUDA(cudaMemcpyAsync(c->clip_off.p, meta.data(), sizeof(int64_t) * 3 * n1, cudaMemcpyHostToDevice, c->stream));
     const int64_t* d_meta = c->clip_off.as<int64_t>();
     c->prof.begin("frontend", c->stream);
-    cudaError_t e = frontend_launch(d_pcm, fmt, d_meta, d_meta + n1, d_meta + 2 * n1, (int)n_clips, preemphasis,
-                                    c->d_tables, d_feats, normalize, c->stream);
+    cudaError_t e = frontend_launch(d_pcm, fmt, d_meta, d_meta + n1, d_meta + 2 * n1, (int)n_clips, fo[n_clips], max_frames, preemphasis,
+                                    c->d_tables, d_feats, normalize, c->stream, &c->launches);
     c->prof.end(c->stream);
     if (e == cudaErrorMisalignedAddress)
         return fail(SB_INVALID_ARGUMENT, "the feature buffer must be 16-byte aligned and the PCM buffer aligned to its sample type");
     SB_CUDA(e);
-    c->launches += 1;
     return SB_OK;
 }
 

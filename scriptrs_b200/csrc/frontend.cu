@@ -6,7 +6,9 @@
 // filterbank, ln(x + 2^-24), per-feature mean / variance normalisation over
 // all frames of the clip.
 //
-// frontend_clip_kernel: one CTA (8 warps) per clip, two CTAs per SM.
+// frontend_clip_kernel: one CTA (8 warps) per clip, two CTAs per SM.  A batch with too few clips to fill the chip has
+// its clips' rows spread over CTAs (the same kernel, a few steps each) and the statistics and normalisation done by
+// frontend_norm_kernel, column block by column block: the same arithmetic in the same order, bit for bit.
 //   rows      The clip is walked 16 frames at a time.  The raw samples of the next 16 frames arrive by cp.async
 //             (16-byte pieces where the clip's placement allows it) while the current ones are transformed; one
 //             pass turns them into pre-emphasised, zero-padded samples (16-bit input is converted here).  Each
@@ -26,6 +28,8 @@
 // different banks.
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "frontend.h"
 #include "frontend_core.cuh"
@@ -85,16 +89,47 @@ struct Sample<int16_t> {
     }
 };
 
-template <typename TIn>
+// (v - mean) / std with the IEEE quotient (frontend.rs:237-239), four columns at a time.  For a divisor in the range
+// below the quotient is formed from the correctly rounded reciprocal and one exact-remainder correction, three
+// instructions, which gives the correctly rounded result (Markstein's correction step; checked against the
+// hardware division on 4e8 operand pairs, all-ones significands included); any other divisor takes __fdiv_rn.
+struct Normaliser {
+    float4 mu, sd, rc;
+    bool fast;
+    static __device__ __forceinline__ bool plain(float d) {
+        const uint32_t b = __float_as_uint(d);
+        return d >= 7.62939453125e-06f && d < 128.0f && (b & 0x7FFFFFu) != 0x7FFFFFu;  // 2^-17 <= d < 2^7
+    }
+    static __device__ __forceinline__ float quot(float x, float d, float r) {
+        const float q = __fmul_rn(x, r);
+        return fmaf(fmaf(-q, d, x), r, q);
+    }
+    __device__ __forceinline__ Normaliser(float4 mean, float4 std) : mu(mean), sd(std) {
+        fast = plain(sd.x) && plain(sd.y) && plain(sd.z) && plain(sd.w);
+        rc = make_float4(__frcp_rn(sd.x), __frcp_rn(sd.y), __frcp_rn(sd.z), __frcp_rn(sd.w));
+    }
+    __device__ __forceinline__ float4 apply(float4 v) const {
+        const float a = __fsub_rn(v.x, mu.x), b = __fsub_rn(v.y, mu.y);
+        const float c = __fsub_rn(v.z, mu.z), d = __fsub_rn(v.w, mu.w);
+        if (fast) return make_float4(quot(a, sd.x, rc.x), quot(b, sd.y, rc.y), quot(c, sd.z, rc.z), quot(d, sd.w, rc.w));
+        return make_float4(__fdiv_rn(a, sd.x), __fdiv_rn(b, sd.y), __fdiv_rn(c, sd.z), __fdiv_rn(d, sd.w));
+    }
+};
+
+// SPLIT: the CTA computes only the log-mel rows of `chunk` steps of its clip (grid: chunks x clips); the statistics
+// and the normalisation are frontend_norm_kernel's.
+template <typename TIn, bool SPLIT>
 __global__ void __launch_bounds__(kThreads, 2)
 frontend_clip_kernel(const TIn* __restrict__ pcm, const int64_t* __restrict__ clip_start,
                      const int64_t* __restrict__ clip_len, const int64_t* __restrict__ frame_off,
-                     float* __restrict__ out, float preemph, const FrontendTables* __restrict__ tables, int normalize) {
+                     float* __restrict__ out, float preemph, const FrontendTables* __restrict__ tables, int normalize,
+                     int chunk) {
+    if constexpr (SPLIT) asm volatile("griddepcontrol.launch_dependents;");  // frontend_norm_kernel waits for this grid itself
     extern __shared__ __align__(16) unsigned char smem_raw[];
     SmemLayout& sm = *reinterpret_cast<SmemLayout*>(smem_raw);
     constexpr int PP = Sample<TIn>::kPerPiece;
 
-    const int clip = blockIdx.x;
+    const int clip = SPLIT ? blockIdx.y : blockIdx.x;
     const int64_t c0 = clip_start[clip];
     const int64_t n = clip_len[clip];
     const int64_t fo = frame_off[clip];
@@ -110,7 +145,10 @@ frontend_clip_kernel(const TIn* __restrict__ pcm, const int64_t* __restrict__ cl
     // pairs with 8-byte loads, so an odd shift + 1 (a clip that starts on an odd sample of the PCM buffer) moves the
     // whole buffer up by one element.
     const int ys_off = (shift + 1) & 1;
-    const int n_steps = (T + kStepFrames - 1) / kStepFrames;
+    const int first_step = SPLIT ? (int)blockIdx.x * chunk : 0;
+    const int all_steps = (T + kStepFrames - 1) / kStepFrames;
+    const int n_steps = SPLIT ? min(all_steps, first_step + chunk) : all_steps;
+    if (SPLIT && first_step >= n_steps) return;
 
     // Raw samples of a step -> shared memory, asynchronously; zero outside the clip (frontend.rs:59-65).
     auto fetch = [&](int step) {
@@ -145,7 +183,7 @@ frontend_clip_kernel(const TIn* __restrict__ pcm, const int64_t* __restrict__ cl
         }
         cp_async_commit();
     };
-    fetch(0);
+    fetch(first_step);
 
     // Tables -> shared memory.
     for (int i = tid; i < kWin; i += kThreads) sm.window[i] = tables->window[i];
@@ -164,7 +202,7 @@ frontend_clip_kernel(const TIn* __restrict__ pcm, const int64_t* __restrict__ cl
             if (f0 + row < T)
                 reinterpret_cast<float4*>(out + (fo + f0 + row) * kMels)[c4] = reinterpret_cast<const float4*>(sm.stage[row])[c4];
         }
-        if (tid < kMels) {
+        if (!SPLIT && tid < kMels) {
             const int rows = min(kStepFrames, T - f0);
             if (rows == kStepFrames) {
 #pragma unroll
@@ -178,10 +216,10 @@ frontend_clip_kernel(const TIn* __restrict__ pcm, const int64_t* __restrict__ cl
     const int half = lane >> 4, p = lane & 15;
     float taps[kMelTapRows];  // this lane's filterbank taps (rows 16 g + p)
     fe::load_mel_taps(p, tables->melw, taps);
-    for (int step = 0; step < n_steps; ++step) {
+    for (int step = first_step; step < n_steps; ++step) {
         cp_async_wait<0>();
         __syncthreads();  // this step's raw samples are in; the previous step's rows are all in the stage
-        if (step > 0) flush(step - 1);
+        if (step > first_step) flush(step - 1);
         // Pre-emphasis (frontend.rs:150-159): y[0] = x[0]; y[i] = x[i] - c * x[i-1], product rounded first; zero outside
         // the clip (the padding is added after the pre-emphasis, frontend.rs:59-65).
         {
@@ -238,7 +276,7 @@ frontend_clip_kernel(const TIn* __restrict__ pcm, const int64_t* __restrict__ cl
     }
     __syncthreads();
     flush(n_steps - 1);
-    if (!normalize) return;
+    if (SPLIT || !normalize) return;
 
     // ---- statistics, frontend.rs:225-236.  Thread c (< 128) owns column c; warp w streams rows of columns
     // 32 w .. 32 w + 31 through its own ring of kRingSlots x kRingRows rows.
@@ -292,24 +330,10 @@ frontend_clip_kernel(const TIn* __restrict__ pcm, const int64_t* __restrict__ cl
         sm.stdv[tid] = __fadd_rn(__fsqrt_rn(variance), 1e-5f);
     }
     __syncthreads();
-    // ---- normalise, frontend.rs:237-239: (v - mean) / std with the IEEE quotient.  For a divisor in the range below
-    // the quotient is formed from the correctly rounded reciprocal and one exact-remainder correction, three
-    // instructions, which gives the correctly rounded result (Markstein's correction step; checked against the
-    // hardware division on 4e8 operand pairs, all-ones significands included); any other divisor takes __fdiv_rn.
+    // ---- normalise, frontend.rs:237-239
     {
         const int c4 = tid & 31;
-        const float4 mu = reinterpret_cast<const float4*>(sm.mean)[c4];
-        const float4 sd = reinterpret_cast<const float4*>(sm.stdv)[c4];
-        auto plain = [](float d) {
-            const uint32_t b = __float_as_uint(d);
-            return d >= 7.62939453125e-06f && d < 128.0f && (b & 0x7FFFFFu) != 0x7FFFFFu;  // 2^-17 <= d < 2^7
-        };
-        const bool fast = plain(sd.x) && plain(sd.y) && plain(sd.z) && plain(sd.w);
-        const float4 rc = make_float4(__frcp_rn(sd.x), __frcp_rn(sd.y), __frcp_rn(sd.z), __frcp_rn(sd.w));
-        auto quot = [](float x, float d, float r) {
-            const float q = __fmul_rn(x, r);
-            return fmaf(fmaf(-q, d, x), r, q);
-        };
+        const Normaliser norm(reinterpret_cast<const float4*>(sm.mean)[c4], reinterpret_cast<const float4*>(sm.stdv)[c4]);
         float4* rows4 = reinterpret_cast<float4*>(out + fo * kMels);
         constexpr int U = 8;
         for (int r0 = tid >> 5; r0 < T; r0 += 8 * U) {
@@ -322,26 +346,130 @@ frontend_clip_kernel(const TIn* __restrict__ pcm, const int64_t* __restrict__ cl
 #pragma unroll
             for (int u = 0; u < U; ++u) {
                 const int r = r0 + 8 * u;
-                if (r < T) {
-                    float4 o;
-                    const float a = __fsub_rn(v[u].x, mu.x), b = __fsub_rn(v[u].y, mu.y);
-                    const float c = __fsub_rn(v[u].z, mu.z), d = __fsub_rn(v[u].w, mu.w);
-                    if (fast) {
-                        o.x = quot(a, sd.x, rc.x);
-                        o.y = quot(b, sd.y, rc.y);
-                        o.z = quot(c, sd.z, rc.z);
-                        o.w = quot(d, sd.w, rc.w);
-                    } else {
-                        o.x = __fdiv_rn(a, sd.x);
-                        o.y = __fdiv_rn(b, sd.y);
-                        o.z = __fdiv_rn(c, sd.z);
-                        o.w = __fdiv_rn(d, sd.w);
-                    }
-                    rows4[(int64_t)r * 32 + c4] = o;
-                }
+                if (r < T) rows4[(int64_t)r * 32 + c4] = norm.apply(v[u]);
             }
         }
     }
+}
+
+// Statistics and normalisation of a clip whose log-mel rows lie in `out`, COLS columns per CTA (grid: column groups x
+// clips).  The T x COLS block of the clip is fetched once into shared memory (cp.async, kNormGroups commit groups, so
+// that the column sums start on the first rows while the others are under way); one warp then walks its columns in
+// frame order, a lane per column, exactly as the one-CTA-per-clip kernel does (frontend.rs:225-236: the order of the
+// sums is part of the result), and all warps normalise.  Bound by the two serial chains of T dependent additions.
+constexpr int kNormGroups = 8;
+template <int COLS>
+__global__ void __launch_bounds__(kThreads)
+frontend_norm_kernel(const int64_t* __restrict__ frame_off, float* __restrict__ out) {
+    extern __shared__ __align__(16) float block[];  // [T][COLS]
+    __shared__ __align__(16) float s_mean[COLS], s_std[COLS];
+    constexpr int PC = COLS / 4;  // 16-byte pieces per row
+    const int clip = blockIdx.y;
+    const int64_t fo = frame_off[clip];
+    const int T = (int)(frame_off[clip + 1] - fo);
+    float* rows = out + fo * kMels + blockIdx.x * COLS;
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int group_rows = (T + kNormGroups - 1) / kNormGroups;
+    asm volatile("griddepcontrol.wait;" ::: "memory");  // the rows of this clip are complete and visible
+#pragma unroll 1
+    for (int g = 0; g < kNormGroups; ++g) {
+        const int r0 = g * group_rows, n = max(0, min(T, r0 + group_rows) - r0) * PC;
+        for (int i = tid; i < n; i += kThreads) {
+            const int r = r0 + i / PC, c = 4 * (i % PC);
+            cp_async16(smem_addr(block + r * COLS + c), rows + (int64_t)r * kMels + c, 16);
+        }
+        cp_async_commit();
+    }
+    float sum = 0.0f;
+    const float* col = block + (lane % COLS);
+    auto add_group = [&](int g) {
+        if (tid >= 32) return;
+        const int r1 = min(T, (g + 1) * group_rows);
+#pragma unroll 16
+        for (int r = g * group_rows; r < r1; ++r) sum = __fadd_rn(sum, col[r * COLS]);
+    };
+    static_assert(kNormGroups == 8, "one wait per group below");
+    cp_async_wait<7>(); __syncthreads(); add_group(0);
+    cp_async_wait<6>(); __syncthreads(); add_group(1);
+    cp_async_wait<5>(); __syncthreads(); add_group(2);
+    cp_async_wait<4>(); __syncthreads(); add_group(3);
+    cp_async_wait<3>(); __syncthreads(); add_group(4);
+    cp_async_wait<2>(); __syncthreads(); add_group(5);
+    cp_async_wait<1>(); __syncthreads(); add_group(6);
+    cp_async_wait<0>(); __syncthreads(); add_group(7);
+    if (tid < 32) {
+        const float mean = __fdiv_rn(sum, (float)T);
+        float acc = 0.0f;
+#pragma unroll 16
+        for (int r = 0; r < T; ++r) {
+            const float d = __fsub_rn(col[r * COLS], mean);
+            acc = __fadd_rn(acc, __fmul_rn(d, d));
+        }
+        // variance / (T - 1); T == 1 divides 0 by 0 and yields NaN exactly as the reference does.
+        const float variance = __fdiv_rn(acc, __fsub_rn((float)T, 1.0f));
+        if (lane < COLS) {
+            s_mean[lane] = mean;
+            s_std[lane] = __fadd_rn(__fsqrt_rn(variance), 1e-5f);
+        }
+    }
+    __syncthreads();
+    static_assert(kThreads % PC == 0, "a thread keeps its columns");
+    const int c4 = tid % PC;
+    const Normaliser norm(reinterpret_cast<const float4*>(s_mean)[c4], reinterpret_cast<const float4*>(s_std)[c4]);
+#pragma unroll 4
+    for (int r = tid / PC; r < T; r += kThreads / PC)
+        *reinterpret_cast<float4*>(rows + (int64_t)r * kMels + 4 * c4) =
+            norm.apply(*reinterpret_cast<const float4*>(block + r * COLS + 4 * c4));
+}
+
+constexpr int kNormMaxSmem = 225 * 1024;
+constexpr int kSplitMaxFrames = kNormMaxSmem / (16 * (int)sizeof(float));  // 3600 (36 s): 16 columns per CTA; half of it: 32
+
+template <int COLS>
+cudaError_t norm_launch(const int64_t* d_frame_off, int n_clips, int max_frames, float* feats, cudaStream_t stream) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(kMels / COLS, n_clips);
+    cfg.blockDim = dim3(kThreads);
+    cfg.dynamicSmemBytes = (size_t)max_frames * COLS * sizeof(float);
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, frontend_norm_kernel<COLS>, d_frame_off, feats);
+}
+
+template <typename TIn>
+cudaError_t launch_format(const TIn* pcm, const int64_t* d_clip_start, const int64_t* d_clip_len, const int64_t* d_frame_off,
+                          int n_clips, int64_t total_frames, int max_frames, float preemph, const FrontendTables* d_tables,
+                          float* feats, bool normalize, cudaStream_t stream, int64_t* launches) {
+    *launches += 1;
+    // One CTA per clip, or the clip's steps and columns spread over the chip.  Measured on clips of 1501 frames
+    // (one-CTA kernel / split, us): 1 clip 304 / 31, 16 clips 304 / 54, 97 ragged clips 307 / 165, 148 clips
+    // 335 / 296, 200 clips 453 / 424, 296 clips 489 / 576; on 3001 frames: 1 clip 598 / 44, 148 clips 663 / 676.  The
+    // one-CTA kernel takes 0.2 us per frame of the longest clip until the SMs are full, the split 1.4 ns per frame in
+    // all, so the line lies where the batch holds about 128 clips' worth of the longest one.  A clip of one or two
+    // steps has nothing to split, and the column blocks of a longer one than kSplitMaxFrames do not fit.
+    const bool split = max_frames > 2 * kStepFrames && max_frames <= kSplitMaxFrames && n_clips <= 65535 &&
+                       total_frames < (int64_t)128 * max_frames;
+    if (!split) {
+        frontend_clip_kernel<TIn, false><<<n_clips, kThreads, sizeof(SmemLayout), stream>>>(
+            pcm, d_clip_start, d_clip_len, d_frame_off, feats, preemph, d_tables, normalize ? 1 : 0, 0);
+        return cudaGetLastError();
+    }
+    const int max_steps = (max_frames + kStepFrames - 1) / kStepFrames;
+    // steps per CTA: four CTAs per resident slot if the batch gives as many (the tables are loaded once per CTA; one
+    // step per CTA is 15 % slower on 97 clips), and a bounded number of CTAs that find their clip already over
+    const int64_t steps = total_frames / kStepFrames + n_clips;
+    const int chunk = (int)std::max(std::min<int64_t>(16, std::max<int64_t>(1, steps / 1184)), (max_steps * (int64_t)n_clips + 16383) / 16384);
+    frontend_clip_kernel<TIn, true><<<dim3((max_steps + chunk - 1) / chunk, n_clips), kThreads, sizeof(SmemLayout), stream>>>(
+        pcm, d_clip_start, d_clip_len, d_frame_off, feats, preemph, d_tables, 0, chunk);
+    cudaError_t e = cudaGetLastError();
+    if (e != cudaSuccess || !normalize) return e;
+    *launches += 1;
+    return max_frames <= kSplitMaxFrames / 2 ? norm_launch<32>(d_frame_off, n_clips, max_frames, feats, stream)
+                                                                   : norm_launch<16>(d_frame_off, n_clips, max_frames, feats, stream);
 }
 
 }  // namespace
@@ -349,27 +477,33 @@ frontend_clip_kernel(const TIn* __restrict__ pcm, const int64_t* __restrict__ cl
 size_t frontend_smem_bytes() { return sizeof(SmemLayout); }
 
 cudaError_t frontend_configure() {
-    cudaError_t e = cudaFuncSetAttribute(frontend_clip_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)sizeof(SmemLayout));
-    if (e != cudaSuccess) return e;
-    return cudaFuncSetAttribute(frontend_clip_kernel<int16_t>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)sizeof(SmemLayout));
+    auto opt_in = [](const void* kernel, size_t bytes) {
+        return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+    };
+    for (const void* k : {(const void*)frontend_clip_kernel<float, false>, (const void*)frontend_clip_kernel<float, true>,
+                          (const void*)frontend_clip_kernel<int16_t, false>, (const void*)frontend_clip_kernel<int16_t, true>}) {
+        const cudaError_t e = opt_in(k, sizeof(SmemLayout));
+        if (e != cudaSuccess) return e;
+    }
+    const cudaError_t e = opt_in((const void*)frontend_norm_kernel<32>, kNormMaxSmem);
+    return e != cudaSuccess ? e : opt_in((const void*)frontend_norm_kernel<16>, kNormMaxSmem);
 }
 
 cudaError_t frontend_launch(const void* pcm, SampleFormat fmt, const int64_t* d_clip_start, const int64_t* d_clip_len,
-                            const int64_t* d_frame_off, int n_clips, float preemph, const FrontendTables* d_tables,
-                            float* feats, bool normalize, cudaStream_t stream) {
+                            const int64_t* d_frame_off, int n_clips, int64_t total_frames, int max_frames, float preemph,
+                            const FrontendTables* d_tables, float* feats, bool normalize, cudaStream_t stream,
+                            int64_t* launches) {
+    int64_t ignored;
+    if (!launches) launches = &ignored;
     if (n_clips <= 0) return cudaSuccess;
     // 16-byte row accesses of the feature matrix and 4- / 2-byte aligned samples
     if ((reinterpret_cast<uintptr_t>(feats) & 15) || (reinterpret_cast<uintptr_t>(pcm) & (fmt == kSampleI16 ? 1 : 3)))
         return cudaErrorMisalignedAddress;
     if (fmt == kSampleI16)
-        frontend_clip_kernel<int16_t><<<n_clips, kThreads, sizeof(SmemLayout), stream>>>(
-            static_cast<const int16_t*>(pcm), d_clip_start, d_clip_len, d_frame_off, feats, preemph, d_tables, normalize ? 1 : 0);
-    else
-        frontend_clip_kernel<float><<<n_clips, kThreads, sizeof(SmemLayout), stream>>>(
-            static_cast<const float*>(pcm), d_clip_start, d_clip_len, d_frame_off, feats, preemph, d_tables, normalize ? 1 : 0);
-    return cudaGetLastError();
+        return launch_format(static_cast<const int16_t*>(pcm), d_clip_start, d_clip_len, d_frame_off, n_clips, total_frames,
+                             max_frames, preemph, d_tables, feats, normalize, stream, launches);
+    return launch_format(static_cast<const float*>(pcm), d_clip_start, d_clip_len, d_frame_off, n_clips, total_frames,
+                         max_frames, preemph, d_tables, feats, normalize, stream, launches);
 }
 
 }  // namespace sb

@@ -50,10 +50,12 @@ enum SampleFormat : int {
 size_t frontend_smem_bytes();
 cudaError_t frontend_configure();
 // Clip i is samples [d_clip_start[i], d_clip_start[i] + d_clip_len[i]) of `pcm` (clips may overlap in the PCM
-// buffer); its features are written at row d_frame_off[i] of feats.  One launch: a CTA per clip computes the
-// log-mel rows and, if `normalize`, the per-feature statistics and the normalised values.
+// buffer); its features are written at row d_frame_off[i] of feats: log-mel rows and, if `normalize`, the per-feature
+// normalisation.  total_frames / max_frames: over all clips / of the longest one.  One launch with a CTA per clip, or
+// two that spread each clip over several CTAs; *launches is advanced by their number.
 cudaError_t frontend_launch(const void* pcm, SampleFormat fmt, const int64_t* d_clip_start, const int64_t* d_clip_len,
-                            const int64_t* d_frame_off, int n_clips, float preemph, const FrontendTables* d_tables,
-                            float* feats, bool normalize, cudaStream_t stream);
+                            const int64_t* d_frame_off, int n_clips, int64_t total_frames, int max_frames, float preemph,
+                            const FrontendTables* d_tables, float* feats, bool normalize, cudaStream_t stream,
+                            int64_t* launches = nullptr);
 
 }  // namespace sb

@@ -28,6 +28,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <algorithm>
 #include <atomic>
 #include <climits>
 #include <cstring>
@@ -114,6 +115,7 @@ extern "C" int32_t sb_frontend_device_noalloc(const float* d_pcm, const int64_t*
     int64_t meta[3 * (kNoAllocMaxClips + 1)] = {};
     int64_t* fo = meta + 2 * n1;
     fo[0] = 0;
+    int max_frames = 0;
     for (int64_t i = 0; i < n_clips; ++i) {
         const int64_t len = clip_offsets[i + 1] - clip_offsets[i];
         if (len <= 0) return fail(SB_EMPTY_AUDIO, "audio input was empty");
@@ -122,6 +124,7 @@ extern "C" int32_t sb_frontend_device_noalloc(const float* d_pcm, const int64_t*
         const int64_t t = frames_for_samples(len);
         if (t > INT32_MAX / 2) return fail(SB_INVALID_ARGUMENT, "clip too long");
         fo[i + 1] = fo[i] + t;
+        max_frames = std::max(max_frames, (int)t);
     }
     if (frame_offsets) std::memcpy(frame_offsets, fo, sizeof(int64_t) * ((size_t)n_clips + 1));
 
@@ -131,7 +134,7 @@ extern "C" int32_t sb_frontend_device_noalloc(const float* d_pcm, const int64_t*
     // pageable source: the runtime has staged the bytes by the time the call returns
     e = cudaMemcpyAsync(d_meta, meta, sizeof(meta), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return cuda_fail(e, "copy of the clip metadata");
-    e = frontend_launch(d_pcm, kSampleF32, d_meta, d_meta + n1, d_meta + 2 * n1, (int)n_clips, preemphasis, d_tables,
+    e = frontend_launch(d_pcm, kSampleF32, d_meta, d_meta + n1, d_meta + 2 * n1, (int)n_clips, fo[n_clips], max_frames, preemphasis, d_tables,
                         d_feats, normalize != 0, st);
     if (e == cudaErrorMisalignedAddress) return fail(SB_INVALID_ARGUMENT, "the feature buffer must be 16-byte aligned");
     if (e != cudaSuccess) return cuda_fail(e, "frontend launch");

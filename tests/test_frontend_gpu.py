@@ -162,3 +162,26 @@ def test_int16_pcm_equals_the_converted_f32_buffer(ctx, fx):
     r = oracle.frontend_extract(pcm32[offs[2]:offs[3]])
     nrm, peak = rel_errors(a[2], r)
     assert nrm <= REL_TOL and peak <= REL_TOL, (nrm, peak)
+
+
+@pytest.mark.parametrize("samples", [32 * 160 - 1, 32 * 160, 239_999, 1800 * 160 - 1, 1800 * 160, 3600 * 160 - 1, 3600 * 160])
+def test_split_clip_equals_one_block_per_clip(ctx, fx, samples):
+    """A lone clip is spread over thread blocks, 130 clips of one length get a block each: the features must be equal bit
+    for bit.  Lengths on both sides of every line of the rule (two steps, 32 and 16 columns per block, longest split)."""
+    import torch
+    import scriptrs_b200 as sb
+
+    n = 130
+    g = torch.Generator(device="cuda").manual_seed(samples)
+    pcm = (torch.randn(n * samples, generator=g, device="cuda") * 0.1).clamp_(-1, 1)
+    t = sb.num_frames(samples)
+    many = torch.full((n * t, 128), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    fx.extract_device(pcm.data_ptr(), np.arange(n + 1, dtype=np.int64) * samples, many.data_ptr())
+    for i in (0, 77, n - 1):
+        one = torch.full((t, 128), float("nan"), device="cuda")
+        torch.cuda.synchronize()
+        fx.extract_device(pcm.data_ptr(), np.array([i * samples, (i + 1) * samples], np.int64), one.data_ptr())
+        ctx.synchronize()
+        assert torch.isfinite(one).all() and torch.equal(one, many[i * t:(i + 1) * t]), (samples, i)
+
