@@ -273,6 +273,7 @@ __device__ void decide_phase(const DecodeState& s, const int* act, int n_act, fl
             const int oi = redi[wv];
             if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
         }
+        if (bi == 0x7fffffff) bi = 0;  // not one comparable logit: the first entry, as a scan from entry 0 leaves it
         float sum = 0.0f;
         for (int i = tid; i < kVocab; i += kThreads) sum += expf(lg[i] - best);
 #pragma unroll

@@ -45,7 +45,6 @@ cudaError_t decode_tc_enc_projection(const DecodeTcWeights& t, const float* d_en
                                      int64_t rows, void* scratch, int sm_count, int* d_error, int64_t* launches,
                                      cudaStream_t st);
 cudaError_t decode_tc_run(const DecodeWeights& w, const DecodeTcWeights& t, const DecodeState& s, int max_steps,
-                          void* scratch_after_enc, int* d_alive, int sm_count, int* d_error, int64_t* launches,
-                          cudaStream_t st);
+                          int64_t enc_rows, void* scratch, int sm_count, int* d_error, int64_t* launches, cudaStream_t st);
 
 }  // namespace sb

@@ -1,24 +1,35 @@
-// TDT greedy decoding with the predictor and joint products on the tensor cores (sm_100a).
+// TDT greedy decoding with the predictor and joint products on the tensor cores (sm_100a): one persistent
+// cooperative kernel for a whole batch.
 //
-// The same state machine as the persistent SIMT kernel in decode.cu (ParakeetModel::greedy_decode and
-// GreedyDecodeState, src/model.rs:64-214), stepped from the host: every iteration runs, for ALL sequences of the
-// batch at once,
-//   GEMM  gates0 = [emb(last_token) | h0] W0^T      cell 0   (c0', h0')
-//   GEMM  gates1 = [h0' | h1] W1^T                  cell 1   (c1', h1')
-//   GEMM  pred   = h1' Wp^T + bp                    joint input  z = relu(enc_proj[frame] + pred)
-//   GEMM  logits = z Wo^T + bo                      decide   (arg-max, confidence, record, commit, advance)
-// The reference runs the predictor only after a token was emitted and otherwise reuses its cached output
-// (src/model.rs:136-160).  Re-running it from the same committed (last_token, h, c) gives the same numbers, so the
-// cache is an optimisation this path does not need: the products are dense over the batch, finished sequences
-// are simply masked in the decide step, and no per-step index lists are built.
+// The state machine is that of the fp32 kernel in decode.cu (ParakeetModel::greedy_decode and GreedyDecodeState,
+// src/model.rs:64-214), and as in the reference the predictor runs only for sequences that emitted a token
+// (src/model.rs:136-160): its output stays cached while a sequence walks over blanks.  One iteration:
+//   A  W_hh0 h0 (+ the table W_ih0 emb(token) + b, one row per vocabulary entry) -> cell 0 -> h0', c0'
+//      W_hh1 h1 -> partial gates of layer 1 (does not need h0', so it shares the phase)
+//   B  W_ih1 h0' + partial -> cell 1 -> h1', c1'
+//   C  W_pred h1' -> z = relu(enc_proj[frame] + pred)
+//   D  W_out z -> logits
+//   E  arg-max, confidence, record, commit, advance; lists of the sequences alive and of those that emitted
+// with a grid-wide barrier between phases; A to C run over the sequences that emitted and are skipped when there are
+// none.  Every product has K = 640.
 //
-// fp32 operands go to the bf16 tensor cores as three-term splits: x = hi + lo with hi = bf16(x), lo = bf16(x - hi),
-// and x . w ~= hi.hi + hi.lo + lo.hi (the dropped terms are below 2^-16 of |x||w|), accumulated in fp32 in tensor
-// memory.  The activation row is stored as [hi | hi | lo] and the weight row as [hi | lo | hi] over a tripled K,
-// so one ordinary bf16 GEMM forms the sum.
+// What bounds it: latency.  A batch of one does 7.6 MMAC per emitted token against 30 MB of weights in L2; a step is a
+// chain of up to five dependent phases of about a microsecond and as many barriers.  Hence mma.sync and not tcgen05:
+// the weight rows are the M side, 16 rows are a tile, and the 444 four-warp groups of the chip share the 65 to 320 tiles
+// of a phase (a 128-row tensor-memory tile would leave most SMs idle and its set-up costs more than the product).  A
+// group keeps its tile's fragments in registers (80 per thread), over all sequences of the phase and, when a phase
+// repeats, over the iterations; the fragments of the phase to come are fetched before the barrier that starts it.
+// Against host-stepped tensor-memory GEMMs over a tripled K (eight kernels an iteration, all sequences in every product):
+// one clip of 188 frames 10.6 -> 1.37 ms, 280 clips of up to 187 frames 14.0 -> 6.7 ms for the whole call.
+//
+// fp32 operands go to the bf16 tensor cores as split sums: x = hi + lo with hi = bf16(x), lo = bf16(x - hi), and
+// x . w ~= hi.hi + hi.lo + lo.hi (the dropped term is below 2^-16 of |x||w|), each of the three in an fp32 accumulator of
+// its own, K in four parts of 160, one per warp, added in a fixed order: a sequence's numbers do not depend on the batch.
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 #include <stdint.h>
+
+#include <algorithm>
 
 #include "context.h"
 #include "decode.h"
@@ -29,14 +40,25 @@ namespace sb {
 namespace {
 
 constexpr int kH = kPredHidden;        // 640
-constexpr int kOutPad = 1152;          // joint output rows padded to a multiple of 128
+static_assert(kH == 640 && kJointDim == 640, "every product of the loop has K = 640");
+constexpr int kGates = 4 * kH;
+constexpr int kKB = kH / 32;           // 20 blocks of 32 k values
+constexpr int kQuadWarps = 4;          // warps that share a tile's K
+constexpr int kWarpKB = kKB / kQuadWarps;
+constexpr int kQuads = 3;              // four-warp groups per CTA
+constexpr int kDecThreads = kQuads * kQuadWarps * 32;
+constexpr int kTileU4 = kKB * 4 * 32;  // uint4 per packed 16-row tile
+constexpr int kLstmTiles = kGates / 16, kPredTiles = kJointDim / 16, kOutTiles = (kJointOut + 15) / 16;
+constexpr int kOutPad = kOutTiles * 16;  // 1040
+constexpr int kPStride = 20;           // floats per column of a partial tile: conflict-free fragment stores
 
 __device__ __forceinline__ void split2(float x, bf16& hi, bf16& lo) {
     hi = __float2bfloat16(x);
     lo = __float2bfloat16(x - __bfloat162float(hi));
 }
 
-// dst [rows x 3 cols] = [hi | hi | lo] of src [rows x cols] (activations).
+// ---------------------------------------------------------------- preparation
+// dst [rows x 3 cols] = [hi | hi | lo] of src [rows x cols] (activations of the encoder projection).
 __global__ void __launch_bounds__(256)
 split_act_kernel(const float* __restrict__ src, bf16* __restrict__ dst, int64_t rows, int cols) {
     const int64_t n = rows * cols;
@@ -52,165 +74,349 @@ split_act_kernel(const float* __restrict__ src, bf16* __restrict__ dst, int64_t 
     }
 }
 
-// dst [rows_pad x 3 (ca + cb)] = [hi | lo | hi] of the rows of [a | b] (weights; b may be null; rows beyond `rows` zero).
+// dst [rows x 3 cols] = [hi | lo | hi] of the rows of src (weights of the encoder projection).
 __global__ void __launch_bounds__(256)
-split_weight_kernel(const float* __restrict__ a, int ca, const float* __restrict__ b, int cb, bf16* __restrict__ dst,
-                    int rows, int rows_pad) {
-    const int k = ca + cb;
-    const int64_t n = (int64_t)rows_pad * k;
+split_weight_kernel(const float* __restrict__ src, int cols, bf16* __restrict__ dst, int rows) {
+    const int64_t n = (int64_t)rows * cols;
     for (int64_t i = (int64_t)blockIdx.x * 256 + threadIdx.x; i < n; i += (int64_t)gridDim.x * 256) {
-        const int r = (int)(i / k), c = (int)(i % k);
-        float x = 0.0f;
-        if (r < rows) x = c < ca ? a[(size_t)r * ca + c] : b[(size_t)r * cb + (c - ca)];
+        const int r = (int)(i / cols), c = (int)(i % cols);
         bf16 hi, lo;
-        split2(x, hi, lo);
-        bf16* d = dst + (size_t)r * 3 * k;
+        split2(src[i], hi, lo);
+        bf16* d = dst + (size_t)r * 3 * cols;
         d[c] = hi;
-        d[k + c] = lo;
-        d[2 * k + c] = hi;
+        d[cols + c] = lo;
+        d[2 * cols + c] = hi;
     }
 }
 
-__global__ void pad_bias_kernel(const float* __restrict__ b, float* __restrict__ out, int n, int n_pad) {
-    const int i = blockIdx.x * 256 + threadIdx.x;
-    if (i < n_pad) out[i] = i < n ? b[i] : 0.0f;
+// Rows of W [rows x 640] in the order of mma.m16n8k16 A fragments: tile, block of 32 k, {hi row g, hi row g + 8, lo row g,
+// lo row g + 8}, lane, eight k values 8 q .. 8 q + 7 (g = lane / 4, q = lane % 4).  The two MMAs of a block take values
+// 0..3 and 4..7 of each lane, which permutes k inside the block; the activations are read with the same permutation.
+// LSTM rows are regrouped so that a tile holds the four gates of four units: row 4 unit + gate.
+__global__ void __launch_bounds__(128)
+pack_fragments_kernel(const float* __restrict__ w, int rows, bool lstm, uint4* __restrict__ dst) {
+    const int tile = blockIdx.x, lane = threadIdx.x & 31, part = threadIdx.x >> 5;
+    const int g = lane >> 2, q = lane & 3;
+    const int r = tile * 16 + g + 8 * (part & 1);
+    const int src = lstm ? (r & 3) * kH + (r >> 2) : r;
+    for (int kb = 0; kb < kKB; ++kb) {
+        __align__(16) bf16 v[8];
+        for (int e = 0; e < 8; ++e) {
+            bf16 hi, lo;
+            split2(src < rows ? w[(size_t)src * kH + kb * 32 + 8 * q + e] : 0.0f, hi, lo);
+            v[e] = part < 2 ? hi : lo;
+        }
+        dst[(size_t)tile * kTileU4 + (kb * 4 + part) * 32 + lane] = *reinterpret_cast<const uint4*>(v);
+    }
 }
 
+// table[token][4 unit + gate] = W_ih0 emb(token) + b0, summed in double: the embedding half of the first cell's gates is a
+// function of the token alone.  grid (tokens, 10), 256 threads.
+__global__ void __launch_bounds__(256)
+token_gates_kernel(const float* __restrict__ embedding, const float* __restrict__ w_ih, const float* __restrict__ b,
+                   float* __restrict__ table) {
+    __shared__ float e[kH];
+    const int token = blockIdx.x, row = blockIdx.y * 256 + threadIdx.x;  // row = gate * 640 + unit
+    for (int i = threadIdx.x; i < kH; i += 256) e[i] = embedding[(size_t)token * kH + i];
+    __syncthreads();
+    double acc = (double)b[row];
+    const float4* w4 = reinterpret_cast<const float4*>(w_ih + (size_t)row * kH);
+    for (int i = 0; i < kH / 4; ++i) {
+        const float4 v = w4[i];
+        acc += (double)v.x * e[4 * i] + (double)v.y * e[4 * i + 1] + (double)v.z * e[4 * i + 2] + (double)v.w * e[4 * i + 3];
+    }
+    table[(size_t)token * kGates + 4 * (row % kH) + row / kH] = (float)acc;
+}
+
+// Bias of layer 1 in the regrouped order, and the joint output bias padded to whole tiles.
+__global__ void bias_kernel(const float* __restrict__ b1, float* __restrict__ b1_out, const float* __restrict__ bo,
+                            float* __restrict__ bo_out) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < kGates) b1_out[4 * (i % kH) + i / kH] = b1[i];
+    if (i < kOutPad) bo_out[i] = i < kJointOut ? bo[i] : 0.0f;
+}
+
+// ---------------------------------------------------------------- the loop
 __device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
 
-// Writes the split row [hi | hi | lo] element c of a K-wide activation row.
-__device__ __forceinline__ void put_split(bf16* row, int k, int c, float x) {
-    bf16 hi, lo;
-    split2(x, hi, lo);
-    row[c] = hi;
-    row[k + c] = hi;
-    row[2 * k + c] = lo;
+__device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+                 : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// First predictor input of every sequence: [emb(blank) | 0].
-__global__ void __launch_bounds__(256)
-dec_init_kernel(const float* __restrict__ embedding, bf16* __restrict__ a0, int n_seq) {
-    const int b = blockIdx.x;
-    bf16* row = a0 + (size_t)b * 3 * 2 * kH;
-    for (int c = threadIdx.x; c < 2 * kH; c += 256)
-        put_split(row, 2 * kH, c, c < kH ? embedding[(size_t)(kVocab - 1) * kH + c] : 0.0f);
+// Everything that the loop writes is read through L2 (ld.cg): the SMs' L1 caches do not see each other's stores.
+struct LoopState {
+    DecodeState s;          // outputs, offsets, frame / token / symbol counters (s.cache_valid holds the parity, see below)
+    DecodeTcWeights w;
+    const float* b_pred;
+    // Candidate and committed predictor states share two slots per sequence: slot `parity` is committed, the other one takes
+    // what the predictor computes from it; emitting a token flips the parity.  [slot][layer][plane hi / lo][n_seq][640]
+    bf16* h;
+    float* c;               // [slot][layer][n_seq][640]
+    bf16* z;                // [plane][n_seq][640] joint input
+    float* part;            // [n_seq][2560] recurrent half of layer 1's gates
+    float* logits;          // [n_seq][1040]
+    // lists of the step (even / odd): sequences alive, sequences whose predictor must run; an entry is b | parity << 30
+    uint32_t *live, *upd;   // [2][n_seq]
+    int* counts;            // [3][2]: alive, must run; three sets used in turn
+    unsigned* barrier;
+    int* error;
+};
+
+constexpr uint32_t kSeqMask = 0x3FFFFFFFu;
+
+enum { kPhaseA = 0, kPhaseB = 1, kPhaseC = 2, kPhaseD = 3 };
+
+struct Fragments {
+    uint4 a[kWarpKB][4];    // {hi g, hi g + 8, lo g, lo g + 8} of this warp's five k blocks
+    const uint4* tile;      // what they hold
+};
+
+__device__ __forceinline__ const uint4* tile_of(const DecodeTcWeights& w, int phase, int t) {
+    if (phase == kPhaseA) return (t < kLstmTiles ? w.hh0 : w.hh1 - (size_t)kLstmTiles * kTileU4) + (size_t)t * kTileU4;
+    const uint4* base = phase == kPhaseB ? w.ih1 : (phase == kPhaseC ? w.pred : w.out);
+    return base + (size_t)t * kTileU4;
+}
+__device__ __forceinline__ constexpr int tiles_of(int phase) {
+    return phase == kPhaseA ? 2 * kLstmTiles : (phase == kPhaseB ? kLstmTiles : (phase == kPhaseC ? kPredTiles : kOutTiles));
 }
 
-// LSTM cell of one layer from the gate pre-activations (bias already added): c' = s(f) c + s(i) tanh(g),
-// h' = s(o) tanh(c').  Layer 0 also writes the next product's input [h0' | h1], layer 1 writes [h1'].
-template <int LAYER>
-__global__ void __launch_bounds__(256)
-dec_cell_kernel(const float* __restrict__ gates, DecodeState s, bf16* __restrict__ a_next, int* __restrict__ step_counter) {
-    const int b = blockIdx.x;
-    if (LAYER == 0 && b == 0 && threadIdx.x == 0) *step_counter += 1;  // one iteration = one pass through these kernels
+__device__ __forceinline__ void fetch_fragments(Fragments& f, const uint4* tile, int qwarp, int lane) {
+    if (f.tile == tile) return;
+    f.tile = tile;
+    const uint4* src = tile + (size_t)qwarp * kWarpKB * 4 * 32 + lane;
+#pragma unroll
+    for (int kb = 0; kb < kWarpKB; ++kb)
+#pragma unroll
+        for (int p = 0; p < 4; ++p) f.a[kb][p] = __ldg(src + (kb * 4 + p) * 32);
+}
+
+// A phase's work is (tiles x groups of 16 sequences), tile-major; each four-warp group takes a contiguous share of it, so
+// that it meets few tiles.
+struct Share {
+    int begin, end, groups;
+};
+__device__ __forceinline__ Share share_of(int phase, int n, int quad) {
+    const int groups = (n + 15) >> 4;
+    const int64_t total = (int64_t)tiles_of(phase) * groups;
+    const int shares = gridDim.x * kQuads, me = quad * gridDim.x + blockIdx.x;
+    return {(int)(total * me / shares), (int)(total * (me + 1) / shares), groups};
+}
+
+template <int PHASE>
+__device__ __forceinline__ void run_phase(const LoopState& L, Fragments& f, const uint32_t* list, int n, int quad, int qwarp, int lane,
+                                          float (*P)[kQuadWarps][16 * kPStride]) {
+    const DecodeState& s = L.s;
+    const Share sh = share_of(PHASE, n, quad);
     const size_t BH = (size_t)s.n_seq * kH;
-    const float* g = gates + (size_t)b * 4 * kH;
-    for (int u = threadIdx.x; u < kH; u += 256) {
-        const size_t idx = (size_t)LAYER * BH + (size_t)b * kH + u;
-        const float cn = sigmoid_f(g[kH + u]) * s.c[idx] + sigmoid_f(g[u]) * tanhf(g[2 * kH + u]);
-        const float hn = sigmoid_f(g[3 * kH + u]) * tanhf(cn);
-        s.c_new[idx] = cn;
-        s.h_new[idx] = hn;
-        if (LAYER == 0) {
-            bf16* row = a_next + (size_t)b * 3 * 2 * kH;
-            put_split(row, 2 * kH, u, hn);
-            put_split(row, 2 * kH, kH + u, s.h[BH + (size_t)b * kH + u]);
-        } else {
-            put_split(a_next + (size_t)b * 3 * kH, kH, u, hn);
+    const int g = lane >> 2, q = lane & 3, qt = qwarp * 32 + lane;
+    int buf = 0;
+    for (int item = sh.begin; item < sh.end; ++item) {
+        const int tile = item / sh.groups, n0 = (item - tile * sh.groups) * 16;
+        const bool rec = PHASE == kPhaseA && tile >= kLstmTiles;  // the recurrent half of layer 1
+        const bool two = n - n0 > 8;
+        // rows of the activations: a column beyond the list repeats the last one and is not stored
+        const uint32_t e0 = __ldcg(list + min(n0 + g, n - 1));
+        const uint32_t e1 = __ldcg(list + min(n0 + 8 + g, n - 1));
+        const uint32_t eo0 = __ldcg(list + min(n0 + (qt >> 4), n - 1)), eo1 = __ldcg(list + min(n0 + 8 + (qt >> 4), n - 1));
+        auto row_of = [&](uint32_t e) -> const bf16* {
+            const size_t b = e & kSeqMask;
+            const int par = e >> 30;
+            if (PHASE == kPhaseD) return L.z + b * kH;
+            const int slot = PHASE == kPhaseA ? par : par ^ 1;
+            const int layer = PHASE == kPhaseA ? (rec ? 1 : 0) : (PHASE == kPhaseB ? 0 : 1);
+            return L.h + (size_t)(slot * 2 + layer) * 2 * BH + b * kH;
+        };
+        const uint4* x0 = reinterpret_cast<const uint4*>(row_of(e0)) + qwarp * kWarpKB * 4 + q;
+        const uint4* x1 = reinterpret_cast<const uint4*>(row_of(e1)) + qwarp * kWarpKB * 4 + q;
+        const size_t plane = BH / 8;  // uint4 from the hi to the lo plane
+        fetch_fragments(f, tile_of(L.w, PHASE, tile), qwarp, lane);
+        // what the epilogue adds, fetched while the product runs: thread qt finishes row qt % 16 of columns qt / 16 (+ 8)
+        const int row = tile * 16 + (qt & 15), r16 = qt & 15;
+        float add[2] = {0.0f, 0.0f}, c_old[2] = {0.0f, 0.0f};
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            const uint32_t e = j ? eo1 : eo0;
+            const size_t b = e & kSeqMask;
+            if (j && !two) continue;
+            if (PHASE == kPhaseA && !rec) {
+                add[j] = __ldg(L.w.token_gates + (size_t)__ldcg(s.last_token + b) * kGates + row);
+                c_old[j] = __ldcg(L.c + (size_t)((e >> 30) * 2) * BH + b * kH + (row >> 2));
+            } else if (PHASE == kPhaseB) {
+                add[j] = __ldcg(L.part + b * kGates + row) + __ldg(L.w.b1 + row);
+                c_old[j] = __ldcg(L.c + (size_t)((e >> 30) * 2 + 1) * BH + b * kH + (row >> 2));
+            } else if (PHASE == kPhaseC) {
+                add[j] = __ldg(L.b_pred + row);
+                c_old[j] = __ldg(s.enc_proj + (size_t)(s.enc_off[b] + __ldcg(s.frame_idx + b)) * kJointDim + row);
+            } else if (PHASE == kPhaseD) {
+                add[j] = __ldg(L.w.b_out + row);
+            }
         }
+        float acc[2][3][4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+#pragma unroll
+            for (int t = 0; t < 3; ++t)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[j][t][i] = 0.0f;
+        auto product = [&](int kb, uint4 xh, uint4 xl, float (&d)[3][4]) {
+            const uint4 h0 = f.a[kb][0], h1 = f.a[kb][1], l0 = f.a[kb][2], l1 = f.a[kb][3];
+            mma_bf16(d[0], h0.x, h1.x, h0.y, h1.y, xh.x, xh.y);
+            mma_bf16(d[1], h0.x, h1.x, h0.y, h1.y, xl.x, xl.y);
+            mma_bf16(d[2], l0.x, l1.x, l0.y, l1.y, xh.x, xh.y);
+            mma_bf16(d[0], h0.z, h1.z, h0.w, h1.w, xh.z, xh.w);
+            mma_bf16(d[1], h0.z, h1.z, h0.w, h1.w, xl.z, xl.w);
+            mma_bf16(d[2], l0.z, l1.z, l0.w, l1.w, xh.z, xh.w);
+        };
+        {
+            uint4 xh[kWarpKB], xl[kWarpKB];
+#pragma unroll
+            for (int kb = 0; kb < kWarpKB; ++kb) {
+                xh[kb] = __ldcg(x0 + kb * 4);
+                xl[kb] = __ldcg(x0 + plane + kb * 4);
+            }
+#pragma unroll
+            for (int kb = 0; kb < kWarpKB; ++kb) product(kb, xh[kb], xl[kb], acc[0]);
+        }
+        if (two) {
+            uint4 xh[kWarpKB], xl[kWarpKB];
+#pragma unroll
+            for (int kb = 0; kb < kWarpKB; ++kb) {
+                xh[kb] = __ldcg(x1 + kb * 4);
+                xl[kb] = __ldcg(x1 + plane + kb * 4);
+            }
+#pragma unroll
+            for (int kb = 0; kb < kWarpKB; ++kb) product(kb, xh[kb], xl[kb], acc[1]);
+        }
+        // partial tiles of the four warps -> shared memory, [column][row]
+        float* mine = P[buf][qwarp];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            if (j && !two) break;
+            float v[4];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) v[i] = acc[j][0][i] + (acc[j][1][i] + acc[j][2][i]);
+            float* o = mine + (8 * j + 2 * q) * kPStride + g;
+            o[0] = v[0];
+            o[kPStride] = v[1];
+            o[8] = v[2];
+            o[kPStride + 8] = v[3];
+        }
+        asm volatile("bar.sync %0, %1;" ::"r"(quad + 1), "r"(kQuadWarps * 32) : "memory");
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            if (j && !two) break;
+            const int at = ((qt >> 4) + 8 * j) * kPStride + r16;
+            const float sum = (P[buf][0][at] + P[buf][1][at]) + (P[buf][2][at] + P[buf][3][at]);
+            const uint32_t e = j ? eo1 : eo0;
+            const size_t b = e & kSeqMask;
+            const bool ok = n0 + (qt >> 4) + 8 * j < n;
+            const float v = sum + add[j];
+            if (PHASE == kPhaseA && rec) {
+                if (ok) __stcg(L.part + b * kGates + (row - kGates), v);
+            } else if (PHASE == kPhaseA || PHASE == kPhaseB) {
+                // the four gates of a unit sit in four neighbouring lanes
+                const int gate = lane & 3, base = lane & ~3;
+                const float act = gate == 2 ? tanhf(v) : sigmoid_f(v);
+                const float gi = __shfl_sync(0xffffffffu, act, base), gf = __shfl_sync(0xffffffffu, act, base + 1);
+                const float gg = __shfl_sync(0xffffffffu, act, base + 2), go = __shfl_sync(0xffffffffu, act, base + 3);
+                const float cn = gf * c_old[j] + gi * gg;
+                const float hn = go * tanhf(cn);
+                if (ok) {
+                    constexpr int layer = PHASE == kPhaseB ? 1 : 0;
+                    const int slot = (int)(e >> 30) ^ 1, unit = row >> 2;
+                    bf16 hi, lo;
+                    split2(hn, hi, lo);
+                    bf16* ho = L.h + (size_t)(slot * 2 + layer) * 2 * BH + b * kH + unit;
+                    if (gate == 0) __stcg(L.c + (size_t)(slot * 2 + layer) * BH + b * kH + unit, cn);
+                    else if (gate == 1) ho[0] = hi;
+                    else if (gate == 2) ho[BH] = lo;
+                }
+            } else if (PHASE == kPhaseC) {
+                if (ok) {
+                    bf16 hi, lo;
+                    split2(fmaxf(c_old[j] + v, 0.0f), hi, lo);
+                    __stcg(s.pred + b * kJointDim + row, v);
+                    L.z[b * kH + row] = hi;
+                    L.z[BH + b * kH + row] = lo;
+                }
+            } else {
+                if (ok) __stcg(L.logits + b * kOutPad + row, v);
+            }
+        }
+        buf ^= 1;  // the other buffer: its readers are behind the barrier above
     }
 }
 
-// z = relu(enc_proj[frame] + pred) -> split row (live sequences only; the others keep a stale, finite row).
-__global__ void __launch_bounds__(256)
-dec_joint_in_kernel(DecodeState s, bf16* __restrict__ a3) {
-    const int b = blockIdx.x;
-    const int frame = s.frame_idx[b];
-    if (frame >= s.enc_len[b]) return;
-    const size_t erow = (size_t)(s.enc_off[b] + frame) * kJointDim;
-    bf16* row = a3 + (size_t)b * 3 * kJointDim;
-    for (int c = threadIdx.x; c < kJointDim; c += 256)
-        put_split(row, kJointDim, c, fmaxf(s.enc_proj[erow + c] + s.pred[(size_t)b * kJointDim + c], 0.0f));
-}
-
-// One CTA per sequence: arg-max, confidence, record, commit, advance (src/model.rs:79-90,180-209), then the next
-// iteration's first predictor input [emb(last_token) | h0].  `alive` receives the number of iterations run so far
-// (step_counter, advanced by the first cell kernel of the iteration) if any sequence still has frames left.
-__global__ void __launch_bounds__(256)
-dec_decide_kernel(DecodeState s, const float* __restrict__ embedding, const float* __restrict__ logits, int ld_logits,
-                  bf16* __restrict__ a0, const int* __restrict__ step_counter, int* __restrict__ alive) {
-    __shared__ float redf[16];
-    __shared__ int redi[8];
-    const int b = blockIdx.x;
-    const int frame = s.frame_idx[b];
-    if (frame >= s.enc_len[b]) return;  // finished (block-uniform)
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+// One warp per sequence: arg-max, confidence, record, commit, advance (src/model.rs:79-90,180-209), the joint input of
+// the next frame where the predictor output stays valid, and the lists of the next step.
+__device__ __forceinline__ void decide(const LoopState& L, uint32_t entry, int lane, uint32_t* next_live, uint32_t* next_upd, int* next_counts) {
+    const DecodeState& s = L.s;
+    const uint32_t b = entry & kSeqMask;
     const size_t BH = (size_t)s.n_seq * kH;
-    const float* lg = logits + (size_t)b * ld_logits;
+    const float* lg = L.logits + (size_t)b * kOutPad;
+    constexpr int kPer = (kVocab + 31) / 32;
+    float v[kPer];
+#pragma unroll
+    for (int i = 0; i < kPer; ++i) v[i] = lane + 32 * i < kVocab ? __ldcg(lg + lane + 32 * i) : -INFINITY;
+    const int frame = __ldcg(s.frame_idx + b), len = s.enc_len[b];
+    const int nsteps = __ldcg(s.n_steps + b), symbols = __ldcg(s.emitted + b);
+    float dl[kDurations];
+#pragma unroll
+    for (int i = 0; i < kDurations; ++i) dl[i] = __ldcg(lg + kVocab + i);
     float best = -INFINITY;
-    int bi = 0x7fffffff;
-    for (int i = tid; i < kVocab; i += 256) {
-        const float v = lg[i];
-        if (v > best) { best = v; bi = i; }  // ascending i per thread: first maximum kept
-    }
+    int token = 0x7fffffff;
+#pragma unroll
+    for (int i = 0; i < kPer; ++i)
+        if (v[i] > best) { best = v[i]; token = lane + 32 * i; }  // ascending index per lane: first maximum kept
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
         const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, bi, o);
-        if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
+        const int oi = __shfl_xor_sync(0xffffffffu, token, o);
+        if (ov > best || (ov == best && oi < token)) { best = ov; token = oi; }
     }
-    if (lane == 0) { redf[warp] = best; redi[warp] = bi; }
-    __syncthreads();
-    best = redf[0];
-    bi = redi[0];
-#pragma unroll
-    for (int wv = 1; wv < 8; ++wv) {
-        const float ov = redf[wv];
-        const int oi = redi[wv];
-        if (ov > best || (ov == best && oi < bi)) { best = ov; bi = oi; }
-    }
+    if (token == 0x7fffffff) token = 0;  // not one comparable logit: the first entry, as a scan from entry 0 leaves it
     float sum = 0.0f;
-    for (int i = tid; i < kVocab; i += 256) sum += expf(lg[i] - best);
+#pragma unroll
+    for (int i = 0; i < kPer; ++i)
+        if (lane + 32 * i < kVocab) sum += expf(v[i] - best);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    if (lane == 0) redf[8 + warp] = sum;
-    __syncthreads();
-    sum = 0.0f;
-#pragma unroll
-    for (int wv = 0; wv < 8; ++wv) sum += redf[8 + wv];
     int dur = 0;
-    {
-        float dv = lg[kVocab];
-        for (int i = 1; i < kDurations; ++i)
-            if (lg[kVocab + i] > dv) { dv = lg[kVocab + i]; dur = i; }
-    }
-    const int token = bi;
-    const int nsteps = s.n_steps[b];
+#pragma unroll
+    for (int i = 1; i < kDurations; ++i)
+        if (dl[i] > dl[0]) { dl[0] = dl[i]; dur = i; }
     if (s.trace && nsteps < s.trace_cap) {
         float* tr = s.trace + ((size_t)b * s.trace_cap + nsteps) * kJointOut;
-        for (int i = tid; i < kJointOut; i += 256) tr[i] = lg[i];
+        for (int i = lane; i < kJointOut; i += 32) tr[i] = __ldcg(lg + i);
     }
     const bool emit = token != kVocab - 1;
-    int emitted = s.emitted[b] + (emit ? 1 : 0);
+    int emitted = symbols + (emit ? 1 : 0);
     int nf = frame;
     if (dur > 0) { nf += dur; emitted = 0; }
     else if (!emit || emitted >= kMaxSymbols) { nf += 1; emitted = 0; }
-    bf16* row = a0 + (size_t)b * 3 * 2 * kH;
-    if (emit) {
-        // commit the predictor state that produced this token (src/model.rs:188-189) and form the next input
-        for (int i = tid; i < kPredLayers * kH; i += 256) {
-            const int l = i / kH, u = i % kH;
-            const size_t idx = (size_t)l * BH + (size_t)b * kH + u;
-            const float hn = s.h_new[idx];
-            s.h[idx] = hn;
-            s.c[idx] = s.c_new[idx];
-            if (l == 0) put_split(row, 2 * kH, kH + u, hn);
+    if (!emit && nf < len) {
+        // the cached predictor output stays valid: joint input of the new frame
+        const float4* en = reinterpret_cast<const float4*>(s.enc_proj + (size_t)(s.enc_off[b] + nf) * kJointDim);
+        const float4* pr = reinterpret_cast<const float4*>(s.pred + (size_t)b * kJointDim);
+#pragma unroll
+        for (int i = 0; i < kJointDim / 128; ++i) {
+            const float4 x = __ldg(en + lane + 32 * i), p = __ldcg(pr + lane + 32 * i);
+            const float zv[4] = {fmaxf(x.x + p.x, 0.0f), fmaxf(x.y + p.y, 0.0f), fmaxf(x.z + p.z, 0.0f), fmaxf(x.w + p.w, 0.0f)};
+            __align__(8) bf16 hi[4], lo[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) split2(zv[e], hi[e], lo[e]);
+            uint2* zo = reinterpret_cast<uint2*>(L.z + (size_t)b * kH) + lane + 32 * i;
+            zo[0] = *reinterpret_cast<const uint2*>(hi);
+            zo[BH / 4] = *reinterpret_cast<const uint2*>(lo);
         }
-        for (int u = tid; u < kH; u += 256) put_split(row, 2 * kH, u, embedding[(size_t)token * kH + u]);
     }
-    if (tid == 0) {
+    if (lane == 0) {
+        // committing the state that produced the token (src/model.rs:188-189) is the flip of the parity
+        const uint32_t next = emit ? entry ^ (1u << 30) : entry;
         if (emit) {
-            const int n = s.n_tokens[b];
+            const int n = __ldcg(s.n_tokens + b);
             if (n < s.max_tokens) {
                 const size_t o = (size_t)b * s.max_tokens + n;
                 s.out_tokens[o] = (uint32_t)token;
@@ -226,59 +432,149 @@ dec_decide_kernel(DecodeState s, const float* __restrict__ embedding, const floa
         s.frame_idx[b] = nf;
         s.emitted[b] = emitted;
         s.n_steps[b] = nsteps + 1;
-        if (nf < s.enc_len[b]) *alive = *step_counter;  // every writer of a step stores the same value
+        if (nf < len) {
+            // the order of a list does not matter: the columns of a product are independent
+            next_live[atomicAdd(next_counts, 1)] = next;
+            if (emit) next_upd[atomicAdd(next_counts + 1, 1)] = next;
+        }
     }
 }
 
-cudaError_t gemm_f32(const bf16* a, const bf16* w, const float* bias, float* out, int M, int N, int K, int sm_count,
-                     int* d_error, cudaStream_t st) {
-    GemmArgs g{};
-    g.a = a;
-    g.w = w;
-    g.bias = bias;
-    g.out = out;
-    g.M = M;
-    g.N = N;
-    g.K = K;
-    g.ldo = N;
-    g.act = kActNone;
-    g.out_mode = kOutF32;
-    g.alpha = 1.0f;
-    g.fp8 = false;
-    return gemm_launch(g, sm_count, d_error, st);
+__global__ void __launch_bounds__(kDecThreads, 1)
+tdt_decode_tc_kernel(const __grid_constant__ LoopState L, int max_steps) {
+    __shared__ __align__(16) float P[kQuads][2][kQuadWarps][16 * kPStride];
+    __shared__ int gave_up;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = warp / kQuadWarps, qwarp = warp % kQuadWarps;
+    const int n_seq = L.s.n_seq;
+    unsigned target = 0;
+    if (tid == 0) gave_up = 0;
+    // Grid-wide barrier over co-resident CTAs (cooperative launch).  The wait is bounded: when it runs out the kernel raises
+    // *error and leaves; the other CTAs then run out of time too.
+    auto grid_barrier = [&]() -> bool {
+        target += gridDim.x;
+        __syncthreads();
+        if (tid == 0) {
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(L.barrier) : "memory");
+            unsigned seen;
+            const long long t0 = clock64();
+            while (true) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(L.barrier) : "memory");
+                if (seen >= target) break;
+                if (clock64() - t0 > 4000000000LL) {
+                    atomicExch(L.error, 1);
+                    gave_up = 1;
+                    break;
+                }
+            }
+        }
+        __syncthreads();
+        return gave_up == 0;
+    };
+    Fragments f;
+    f.tile = nullptr;
+    auto fetch_ahead = [&](int phase, int n) {
+        const Share sh = share_of(phase, n, quad);
+        if (sh.begin < sh.end) fetch_fragments(f, tile_of(L.w, phase, sh.begin / sh.groups), qwarp, lane);
+    };
+    for (int step = 0; step < max_steps; ++step) {
+        const uint32_t* live = L.live + (size_t)(step & 1) * n_seq;
+        const uint32_t* upd = L.upd + (size_t)(step & 1) * n_seq;
+        const int2 n = __ldcg(reinterpret_cast<const int2*>(L.counts) + step % 3);  // {alive, predictor must run}
+        if (n.x == 0) break;
+        if (n.y > 0) {
+            run_phase<kPhaseA>(L, f, upd, n.y, quad, qwarp, lane, P[quad]);
+            fetch_ahead(kPhaseB, n.y);
+            if (!grid_barrier()) return;
+            run_phase<kPhaseB>(L, f, upd, n.y, quad, qwarp, lane, P[quad]);
+            fetch_ahead(kPhaseC, n.y);
+            if (!grid_barrier()) return;
+            run_phase<kPhaseC>(L, f, upd, n.y, quad, qwarp, lane, P[quad]);
+            fetch_ahead(kPhaseD, n.x);
+            if (!grid_barrier()) return;
+        }
+        run_phase<kPhaseD>(L, f, live, n.x, quad, qwarp, lane, P[quad]);
+        // the counters of the step after the next were last read when this step's predecessor began
+        if (blockIdx.x == 0 && tid == 0) __stcg(reinterpret_cast<int2*>(L.counts) + (step + 2) % 3, make_int2(0, 0));
+        if (!grid_barrier()) return;
+        uint32_t* next_live = L.live + (size_t)((step + 1) & 1) * n_seq;
+        uint32_t* next_upd = L.upd + (size_t)((step + 1) & 1) * n_seq;
+        int* next_counts = L.counts + 2 * ((step + 1) % 3);
+        for (int i = warp * gridDim.x + blockIdx.x; i < n.x; i += gridDim.x * (kDecThreads / 32))
+            decide(L, __ldcg(live + i), lane, next_live, next_upd, next_counts);
+        if (!grid_barrier()) return;
+    }
 }
+
+// Lists of the first step: every sequence with frames is alive and its predictor must run (blank, zero state).
+__global__ void dec_init_kernel(LoopState L) {
+    for (int b = blockIdx.x * 256 + threadIdx.x; b < L.s.n_seq; b += gridDim.x * 256)
+        if (L.s.enc_len[b] > 0) {
+            L.live[atomicAdd(L.counts, 1)] = b;
+            L.upd[atomicAdd(L.counts + 1, 1)] = b;
+        }
+}
+
+constexpr size_t align256(size_t n) { return (n + 255) / 256 * 256; }
+
+struct ScratchLayout {
+    size_t h, c, z, part, logits, live, upd, counts, barrier, total;
+    explicit ScratchLayout(int n_seq) {
+        const size_t B = (size_t)n_seq;
+        size_t at = 0;
+        auto take = [&](size_t bytes) { const size_t o = at; at += align256(bytes); return o; };
+        // zeroed at the start: states, counters, barrier
+        h = take(8 * B * kH * sizeof(bf16));
+        c = take(4 * B * kH * sizeof(float));
+        counts = take(6 * sizeof(int));
+        barrier = take(sizeof(unsigned));
+        z = take(2 * B * kH * sizeof(bf16));
+        part = take(B * kGates * sizeof(float));
+        logits = take(B * kOutPad * sizeof(float));
+        live = take(2 * B * sizeof(uint32_t));
+        upd = take(2 * B * sizeof(uint32_t));
+        total = at;
+    }
+};
 
 }  // namespace
 
+constexpr size_t kPackedTiles = 3 * kLstmTiles + kPredTiles + kOutTiles;
+
 size_t decode_tc_weight_bytes() {
-    return sizeof(bf16) * 3 * ((size_t)2 * 4 * kH * 2 * kH + (size_t)kJointDim * kH + (size_t)kOutPad * kJointDim +
-                               (size_t)kJointDim * kDModel) + sizeof(float) * kOutPad;
+    return sizeof(uint4) * kPackedTiles * kTileU4 + sizeof(float) * ((size_t)kVocab * kGates + kGates + kOutPad) +
+           sizeof(bf16) * 3 * (size_t)kJointDim * kDModel;
 }
 
 cudaError_t decode_tc_prepare(const DecodeWeights& w, const float* w_enc, DecodeTcWeights* t, void* storage,
                               cudaStream_t st) {
-    bf16* p = reinterpret_cast<bf16*>(storage);
-    const size_t G = (size_t)4 * kH * kH;
-    t->w0 = p; p += (size_t)4 * kH * 3 * 2 * kH;
-    t->w1 = p; p += (size_t)4 * kH * 3 * 2 * kH;
-    t->wp = p; p += (size_t)kJointDim * 3 * kH;
-    t->wo = p; p += (size_t)kOutPad * 3 * kJointDim;
-    t->wenc = p; p += (size_t)kJointDim * 3 * kDModel;
-    t->b_out = reinterpret_cast<float*>(p);
-    split_weight_kernel<<<1024, 256, 0, st>>>(w.w_ih, kH, w.w_hh, kH, t->w0, 4 * kH, 4 * kH);
-    split_weight_kernel<<<1024, 256, 0, st>>>(w.w_ih + G, kH, w.w_hh + G, kH, t->w1, 4 * kH, 4 * kH);
-    split_weight_kernel<<<256, 256, 0, st>>>(w.w_pred, kH, nullptr, 0, t->wp, kJointDim, kJointDim);
-    split_weight_kernel<<<512, 256, 0, st>>>(w.w_out, kJointDim, nullptr, 0, t->wo, kJointOut, kOutPad);
-    split_weight_kernel<<<512, 256, 0, st>>>(w_enc, kDModel, nullptr, 0, t->wenc, kJointDim, kJointDim);
-    pad_bias_kernel<<<(kOutPad + 255) / 256, 256, 0, st>>>(w.b_out, t->b_out, kJointOut, kOutPad);
+    uint4* p = reinterpret_cast<uint4*>(storage);
+    const size_t G = (size_t)kGates * kH;
+    auto pack = [&](const float* src, int rows, int tiles, bool lstm) -> const uint4* {
+        uint4* dst = p;
+        pack_fragments_kernel<<<tiles, 128, 0, st>>>(src, rows, lstm, dst);
+        p += (size_t)tiles * kTileU4;
+        return dst;
+    };
+    t->hh0 = pack(w.w_hh, kGates, kLstmTiles, true);
+    t->ih1 = pack(w.w_ih + G, kGates, kLstmTiles, true);
+    t->hh1 = pack(w.w_hh + G, kGates, kLstmTiles, true);
+    t->pred = pack(w.w_pred, kJointDim, kPredTiles, false);
+    t->out = pack(w.w_out, kJointOut, kOutTiles, false);
+    float* q = reinterpret_cast<float*>(p);
+    t->token_gates = q;
+    token_gates_kernel<<<dim3(kVocab, kGates / 256), 256, 0, st>>>(w.embedding, w.w_ih, w.b_gates, q);
+    q += (size_t)kVocab * kGates;
+    t->b1 = q;
+    t->b_out = q + kGates;
+    bias_kernel<<<(kGates + 255) / 256, 256, 0, st>>>(w.b_gates + kGates, q, w.b_out, q + kGates);
+    q += kGates + kOutPad;
+    t->wenc = reinterpret_cast<bf16*>(q);
+    split_weight_kernel<<<512, 256, 0, st>>>(w_enc, kDModel, t->wenc, kJointDim);
     return cudaGetLastError();
 }
 
 size_t decode_tc_scratch_bytes(int64_t enc_rows, int n_seq) {
-    const size_t B = (size_t)n_seq;
-    return sizeof(bf16) * ((size_t)enc_rows * 3 * kDModel) +
-           sizeof(bf16) * B * (3 * 2 * kH * 2 + 3 * kH + 3 * kJointDim) +
-           sizeof(float) * B * (4 * kH + kOutPad) + 256;
+    return align256(sizeof(bf16) * (size_t)enc_rows * 3 * kDModel) + ScratchLayout(n_seq).total;
 }
 
 // enc_proj [rows x 640] = enc [rows x 1024] W_enc^T + b_enc through the split product.
@@ -288,74 +584,49 @@ cudaError_t decode_tc_enc_projection(const DecodeTcWeights& t, const float* d_en
     if (rows <= 0) return cudaSuccess;
     bf16* a = reinterpret_cast<bf16*>(scratch);
     split_act_kernel<<<2048, 256, 0, st>>>(d_enc, a, rows, kDModel);
-    cudaError_t e = gemm_f32(a, t.wenc, b_enc, d_proj, (int)rows, kJointDim, 3 * kDModel, sm_count, d_error, st);
+    GemmArgs g{};
+    g.a = a;
+    g.w = t.wenc;
+    g.bias = b_enc;
+    g.out = d_proj;
+    g.M = (int)rows;
+    g.N = kJointDim;
+    g.K = 3 * kDModel;
+    g.ldo = kJointDim;
+    g.act = kActNone;
+    g.out_mode = kOutF32;
+    g.alpha = 1.0f;
+    g.fp8 = false;
+    const cudaError_t e = gemm_launch(g, sm_count, d_error, st);
     *launches += 2;
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 
-// Runs the greedy loop for s.n_seq sequences.  One iteration (four products, four element-wise kernels) is
-// captured into a CUDA graph once per call and replayed; the host launches `check_every` iterations at a time and
-// then reads the `alive` word (d_alive[0]; d_alive[1] is the device-side iteration counter).  Iterations launched
-// after the last sequence finished find nothing to do.
+// Runs the greedy loop for s.n_seq sequences (the integer state is set up by the caller).
 cudaError_t decode_tc_run(const DecodeWeights& w, const DecodeTcWeights& t, const DecodeState& s, int max_steps,
-                          void* scratch_after_enc, int* d_alive, int sm_count, int* d_error, int64_t* launches,
-                          cudaStream_t st) {
-    const int B = s.n_seq;
-    bf16* a0 = reinterpret_cast<bf16*>(scratch_after_enc);
-    bf16* a1 = a0 + (size_t)B * 3 * 2 * kH;
-    bf16* a2 = a1 + (size_t)B * 3 * 2 * kH;
-    bf16* a3 = a2 + (size_t)B * 3 * kH;
-    float* gates = reinterpret_cast<float*>(a3 + (size_t)B * 3 * kJointDim);
-    float* logits = gates + (size_t)B * 4 * kH;
-    int* d_step = d_alive + 1;
-    cudaError_t e = cudaMemsetAsync(d_alive, 0, 2 * sizeof(int), st);
+                          int64_t enc_rows, void* scratch, int sm_count, int* d_error, int64_t* launches, cudaStream_t st) {
+    char* base = static_cast<char*>(scratch) + align256(sizeof(bf16) * (size_t)enc_rows * 3 * kDModel);
+    const ScratchLayout lay(s.n_seq);
+    LoopState L{};
+    L.s = s;
+    L.w = t;
+    L.b_pred = w.b_pred;
+    L.h = reinterpret_cast<bf16*>(base + lay.h);
+    L.c = reinterpret_cast<float*>(base + lay.c);
+    L.z = reinterpret_cast<bf16*>(base + lay.z);
+    L.part = reinterpret_cast<float*>(base + lay.part);
+    L.logits = reinterpret_cast<float*>(base + lay.logits);
+    L.live = reinterpret_cast<uint32_t*>(base + lay.live);
+    L.upd = reinterpret_cast<uint32_t*>(base + lay.upd);
+    L.counts = reinterpret_cast<int*>(base + lay.counts);
+    L.barrier = reinterpret_cast<unsigned*>(base + lay.barrier);
+    L.error = d_error;
+    cudaError_t e = cudaMemsetAsync(base, 0, lay.z, st);
     if (e != cudaSuccess) return e;
-    dec_init_kernel<<<B, 256, 0, st>>>(w.embedding, a0, B);
-    *launches += 1;
-
-    auto iteration = [&]() -> cudaError_t {
-        cudaError_t r = gemm_f32(a0, t.w0, w.b_gates, gates, B, 4 * kH, 3 * 2 * kH, sm_count, d_error, st);
-        if (r != cudaSuccess) return r;
-        dec_cell_kernel<0><<<B, 256, 0, st>>>(gates, s, a1, d_step);
-        r = gemm_f32(a1, t.w1, w.b_gates + 4 * kH, gates, B, 4 * kH, 3 * 2 * kH, sm_count, d_error, st);
-        if (r != cudaSuccess) return r;
-        dec_cell_kernel<1><<<B, 256, 0, st>>>(gates, s, a2, d_step);
-        r = gemm_f32(a2, t.wp, w.b_pred, s.pred, B, kJointDim, 3 * kH, sm_count, d_error, st);
-        if (r != cudaSuccess) return r;
-        dec_joint_in_kernel<<<B, 256, 0, st>>>(s, a3);
-        r = gemm_f32(a3, t.wo, t.b_out, logits, B, kOutPad, 3 * kJointDim, sm_count, d_error, st);
-        if (r != cudaSuccess) return r;
-        dec_decide_kernel<<<B, 256, 0, st>>>(s, w.embedding, logits, kOutPad, a0, d_step, d_alive);
-        return cudaGetLastError();
-    };
-
-    // capture one iteration; on any capture problem fall back to plain launches
-    cudaGraph_t graph = nullptr;
-    cudaGraphExec_t exec = nullptr;
-    if (cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
-        const cudaError_t ce = iteration();
-        const cudaError_t ee = cudaStreamEndCapture(st, &graph);
-        if (ce != cudaSuccess || ee != cudaSuccess || !graph ||
-            cudaGraphInstantiate(&exec, graph, nullptr, nullptr, 0) != cudaSuccess)
-            exec = nullptr;
-    }
-    (void)cudaGetLastError();  // a failed capture leaves a sticky-free error code behind
-
-    constexpr int check_every = 8;
-    int h_alive = 0;
-    for (int step = 0; step < max_steps; ++step) {
-        e = exec ? cudaGraphLaunch(exec, st) : iteration();
-        if (e != cudaSuccess) break;
-        *launches += 8;
-        if ((step + 1) % check_every == 0 || step + 1 == max_steps) {
-            e = cudaMemcpyAsync(&h_alive, d_alive, sizeof(int), cudaMemcpyDeviceToHost, st);
-            if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-            if (e != cudaSuccess) break;
-            if (h_alive < step + 1) break;  // no sequence had frames left after the last launched iteration
-        }
-    }
-    if (exec) cudaGraphExecDestroy(exec);
-    if (graph) cudaGraphDestroy(graph);
+    dec_init_kernel<<<std::min(32, (s.n_seq + 255) / 256), 256, 0, st>>>(L);
+    void* args[] = {&L, &max_steps};
+    e = cudaLaunchCooperativeKernel((const void*)tdt_decode_tc_kernel, dim3(sm_count), dim3(kDecThreads), args, 0, st);
+    *launches += 2;
     return e != cudaSuccess ? e : cudaGetLastError();
 }
 

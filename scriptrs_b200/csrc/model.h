@@ -54,14 +54,14 @@ struct LayerWeights {
     float ff1_wn, ff1_bmax, ff2_wn, ff2_bmax;
 };
 
-// Split-bf16 copies of the predictor / joint weights for the tensor-core path (decode_tc.cu): every row is
-// [hi | lo | hi] over a tripled K; the joint output matrix and bias are padded to 1152 rows.
+// Predictor / joint weights for the tensor-core decoder (decode_tc.cu): split bf16 in the order of its MMA fragments, the
+// embedding half of the first cell's gates as a table over the vocabulary, and the encoder projection as split rows.
 struct DecodeTcWeights {
-    bf16 *w0 = nullptr, *w1 = nullptr;  // [2560 x 3 * 1280]  ([W_ih | W_hh] of each LSTM layer)
-    bf16* wp = nullptr;                 // [640 x 3 * 640]
-    bf16* wo = nullptr;                 // [1152 x 3 * 640]
-    bf16* wenc = nullptr;               // [640 x 3 * 1024]
-    float* b_out = nullptr;             // [1152]
+    const uint4 *hh0 = nullptr, *ih1 = nullptr, *hh1 = nullptr;  // 160 tiles of 16 gate rows each
+    const uint4 *pred = nullptr, *out = nullptr;                 // 40 and 65 tiles
+    const float* token_gates = nullptr;                          // [1025 x 2560] W_ih0 emb(token) + b0
+    const float *b1 = nullptr, *b_out = nullptr;                 // [2560], [1040]
+    bf16* wenc = nullptr;                                        // [640 x 3 * 1024], rows [hi | lo | hi]
 };
 
 struct Model {
@@ -82,7 +82,7 @@ struct Model {
     float *embedding = nullptr, *w_ih = nullptr, *w_hh = nullptr, *b_gates = nullptr;  // b_gates = b_ih + b_hh
     bf16* enc_proj_w = nullptr;  // [640 x 1024] bf16 copy for the tensor-core projection
     float *w_enc = nullptr, *b_enc = nullptr, *w_pred = nullptr, *b_pred = nullptr, *w_out = nullptr, *b_out = nullptr;
-    DecodeTcWeights tc;  // split-bf16 copies for the tensor-core decoder
+    DecodeTcWeights tc;  // operands of the tensor-core decoder
     std::vector<void*> allocations;
 };
 

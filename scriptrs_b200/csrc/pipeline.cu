@@ -75,7 +75,7 @@ int32_t tdt_decode(sb_ctx* c, const float* d_enc, const int64_t* enc_offsets, in
         const size_t n_f = 8 * BH + 2 * (size_t)n * kJointDim + (size_t)n * kJointOut;
         SB_CUDA(ws.floats.ensure(n_f * sizeof(float)));
         float* df = ws.floats.as<float>();
-        SB_CUDA(cudaMemsetAsync(df, 0, 4 * BH * sizeof(float), st));  // h = c = 0 (model.rs:114-115)
+        if (c->simt_decode) SB_CUDA(cudaMemsetAsync(df, 0, 4 * BH * sizeof(float), st));  // h = c = 0 (model.rs:114-115)
         SB_CUDA(ws.enc_proj.ensure((size_t)std::max<int64_t>(rows, 1) * kJointDim * sizeof(float)));
         SB_CUDA(ws.out_tok.ensure((size_t)n * max_tokens * sizeof(uint32_t)));
         SB_CUDA(ws.out_frm.ensure((size_t)n * max_tokens * sizeof(int)));
@@ -135,10 +135,8 @@ int32_t tdt_decode(sb_ctx* c, const float* d_enc, const int64_t* enc_offsets, in
         s.timing = d_timing;
         const int max_steps = (kMaxSymbols + 1) * max_len + 2;
         if (max_len > 0 && tc) {
-            // the per-sequence buffers follow the split encoder rows in the scratch area
-            char* after_enc = static_cast<char*>(ws.tc.p) + sizeof(bf16) * (size_t)rows * 3 * kDModel;
             c->prof.begin("tdt_decode_tc", st);
-            SB_CUDA(decode_tc_run(w, m.tc, s, max_steps, after_enc, di + 8 * n + 1, c->sm_count, c->d_error, &c->launches, st));
+            SB_CUDA(decode_tc_run(w, m.tc, s, max_steps, rows, ws.tc.p, c->sm_count, c->d_error, &c->launches, st));
             c->prof.end(st);
         } else if (max_len > 0) {
             c->prof.begin("tdt_decode", st);
