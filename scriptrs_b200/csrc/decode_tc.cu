@@ -156,7 +156,10 @@ struct LoopState {
     float* c;               // [slot][layer][n_seq][640]
     bf16* z;                // [plane][n_seq][640] joint input
     float* part;            // [n_seq][2560] recurrent half of layer 1's gates
-    float* logits;          // [n_seq][1040]
+    // Every tile of 16 joint outputs leaves {largest token logit, its index, sum of exp(logit - largest)} per sequence; the
+    // last tile also leaves its logits (the blank and the durations).  Two sets, used in turn.
+    float4* stat;           // [2][n_seq][65]
+    float* tail;            // [2][n_seq][16]
     // lists of the step (even / odd): sequences alive, sequences whose predictor must run; an entry is b | parity << 30
     uint32_t *live, *upd;   // [2][n_seq]
     int* counts;            // [3][2]: alive, must run; three sets used in turn
@@ -204,9 +207,130 @@ __device__ __forceinline__ Share share_of(int phase, int n, int quad) {
     return {(int)(total * me / shares), (int)(total * (me + 1) / shares), groups};
 }
 
+// Products of a warp's five k blocks: hi.hi, hi.lo and lo.hi into accumulators of their own.
+__device__ __forceinline__ void load_x(uint4 (&xh)[kWarpKB], uint4 (&xl)[kWarpKB], const uint4* x, size_t plane) {
+#pragma unroll
+    for (int kb = 0; kb < kWarpKB; ++kb) {
+        xh[kb] = __ldcg(x + kb * 4);
+        xl[kb] = __ldcg(x + plane + kb * 4);
+    }
+}
+__device__ __forceinline__ void product(const Fragments& f, const uint4 (&xh)[kWarpKB], const uint4 (&xl)[kWarpKB], float (&v)[4]) {
+    float d[3][4] = {};
+#pragma unroll
+    for (int kb = 0; kb < kWarpKB; ++kb) {
+        const uint4 h0 = f.a[kb][0], h1 = f.a[kb][1], l0 = f.a[kb][2], l1 = f.a[kb][3];
+        mma_bf16(d[0], h0.x, h1.x, h0.y, h1.y, xh[kb].x, xh[kb].y);
+        mma_bf16(d[1], h0.x, h1.x, h0.y, h1.y, xl[kb].x, xl[kb].y);
+        mma_bf16(d[2], l0.x, l1.x, l0.y, l1.y, xh[kb].x, xh[kb].y);
+        mma_bf16(d[0], h0.z, h1.z, h0.w, h1.w, xh[kb].z, xh[kb].w);
+        mma_bf16(d[1], h0.z, h1.z, h0.w, h1.w, xl[kb].z, xl[kb].w);
+        mma_bf16(d[2], l0.z, l1.z, l0.w, l1.w, xh[kb].z, xh[kb].w);
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = d[0][i] + (d[1][i] + d[2][i]);
+}
+// A warp's partial tile (16 rows x 8 columns from column 8 j) -> shared memory, [column][row].
+__device__ __forceinline__ void store_partial(float* mine, int j, int lane, const float (&v)[4]) {
+    float* o = mine + (8 * j + 2 * (lane & 3)) * kPStride + (lane >> 2);
+    o[0] = v[0];
+    o[kPStride] = v[1];
+    o[8] = v[2];
+    o[kPStride + 8] = v[3];
+}
+__device__ __forceinline__ void quad_barrier(int quad) {
+    asm volatile("bar.sync %0, %1;" ::"r"(quad + 1), "r"(kQuadWarps * 32) : "memory");
+}
+__device__ __forceinline__ float sum_partials(float (*P)[16 * kPStride], int at) { return (P[0][at] + P[1][at]) + (P[2][at] + P[3][at]); }
+
+// One LSTM unit: its four gates (i, f, g, o) sit in four neighbouring lanes, pre-activation v.
+__device__ __forceinline__ void cell(float v, float c_old, int lane, float& cn, float& hn) {
+    const int base = lane & ~3;
+    const float act = (lane & 3) == 2 ? tanhf(v) : sigmoid_f(v);
+    const float gi = __shfl_sync(0xffffffffu, act, base), gf = __shfl_sync(0xffffffffu, act, base + 1);
+    const float gg = __shfl_sync(0xffffffffu, act, base + 2), go = __shfl_sync(0xffffffffu, act, base + 3);
+    cn = gf * c_old + gi * gg;
+    hn = go * tanhf(cn);
+}
+// The same sixteen lanes that hold a column of a joint output tile reduce it (row = lane % 16 of the tile).
+__device__ __forceinline__ void tile_stat(float v, int tile, int row, int lane, bool ok, float4* stat, float* tail) {
+    float m = row < kVocab ? v : -INFINITY;
+    int idx = row;
+    const float own = m;
+    if (!(m > -INFINITY)) { m = -INFINITY; idx = 0x7fffffff; }  // nothing to compare with (not a number counts in the sum only)
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, m, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, idx, o);
+        if (ov > m || (ov == m && oi < idx)) { m = ov; idx = oi; }
+    }
+    float e = own == -INFINITY ? 0.0f : expf(own - m);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) e += __shfl_xor_sync(0xffffffffu, e, o);
+    if (!ok) return;
+    if ((lane & 15) == 0) __stcg(stat + tile, make_float4(m, __int_as_float(idx), e, 0.0f));
+    if (tile == kOutTiles - 1) __stcg(tail + (lane & 15), v);
+}
+
+struct Decision {
+    int token, dur;
+    float conf;
+};
+// One warp: arg-max over the tiles (ties to the lowest index), confidence = largest softmax, arg-max of the durations.
+__device__ __forceinline__ Decision decide_tokens(const float4* stat, const float* tail, int lane) {
+    static_assert(kOutTiles == 65 && kVocab == 64 * 16 + 1, "the last tile holds the blank and the durations");
+    float4 t[3];
+    t[0] = __ldcg(stat + lane);
+    t[1] = __ldcg(stat + 32 + lane);
+    t[2] = lane == 0 ? __ldcg(stat + 64) : make_float4(-INFINITY, __int_as_float(0x7fffffff), 0.0f, 0.0f);
+    float dl[kDurations];
+#pragma unroll
+    for (int i = 0; i < kDurations; ++i) dl[i] = __ldcg(tail + 1 + i);
+    float best = t[0].x;
+    int token = __float_as_int(t[0].y);
+#pragma unroll
+    for (int i = 1; i < 3; ++i)
+        if (t[i].x > best) { best = t[i].x; token = __float_as_int(t[i].y); }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
+        const int oi = __shfl_xor_sync(0xffffffffu, token, o);
+        if (ov > best || (ov == best && oi < token)) { best = ov; token = oi; }
+    }
+    if (token == 0x7fffffff) token = 0;  // not one comparable logit: the first entry, as a scan from entry 0 leaves it
+    float sum = 0.0f;
+#pragma unroll
+    for (int i = 0; i < 3; ++i)
+        if (t[i].z != 0.0f) sum += t[i].z * expf(t[i].x - best);
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
+    int dur = 0;
+#pragma unroll
+    for (int i = 1; i < kDurations; ++i)
+        if (dl[i] > dl[0]) { dl[0] = dl[i]; dur = i; }
+    return {token, dur, best > -INFINITY ? 1.0f / sum : NAN};
+}
+// Frame and symbol counter after a decision (src/model.rs:196-209).
+__device__ __forceinline__ void advance(bool emit, int dur, int& frame, int& symbols) {
+    symbols += emit ? 1 : 0;
+    if (dur > 0) { frame += dur; symbols = 0; }
+    else if (!emit || symbols >= kMaxSymbols) { frame += 1; symbols = 0; }
+}
+__device__ __forceinline__ void record(const DecodeState& s, uint32_t b, int n, const Decision& d, int frame) {
+    if (n < s.max_tokens) {
+        const size_t o = (size_t)b * s.max_tokens + n;
+        s.out_tokens[o] = (uint32_t)d.token;
+        s.out_frames[o] = frame;
+        s.out_durs[o] = d.dur;
+        s.out_conf[o] = d.conf;
+    } else {
+        atomicExch(s.overflow, 1);
+    }
+}
+
 template <int PHASE>
 __device__ __forceinline__ void run_phase(const LoopState& L, Fragments& f, const uint32_t* list, int n, int quad, int qwarp, int lane,
-                                          float (*P)[kQuadWarps][16 * kPStride]) {
+                                          float (*P)[kQuadWarps][16 * kPStride], size_t set = 0) {
     const DecodeState& s = L.s;
     const Share sh = share_of(PHASE, n, quad);
     const size_t BH = (size_t)s.n_seq * kH;
@@ -253,62 +377,25 @@ __device__ __forceinline__ void run_phase(const LoopState& L, Fragments& f, cons
                 add[j] = __ldg(L.w.b_out + row);
             }
         }
-        float acc[2][3][4];
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-#pragma unroll
-            for (int t = 0; t < 3; ++t)
-#pragma unroll
-                for (int i = 0; i < 4; ++i) acc[j][t][i] = 0.0f;
-        auto product = [&](int kb, uint4 xh, uint4 xl, float (&d)[3][4]) {
-            const uint4 h0 = f.a[kb][0], h1 = f.a[kb][1], l0 = f.a[kb][2], l1 = f.a[kb][3];
-            mma_bf16(d[0], h0.x, h1.x, h0.y, h1.y, xh.x, xh.y);
-            mma_bf16(d[1], h0.x, h1.x, h0.y, h1.y, xl.x, xl.y);
-            mma_bf16(d[2], l0.x, l1.x, l0.y, l1.y, xh.x, xh.y);
-            mma_bf16(d[0], h0.z, h1.z, h0.w, h1.w, xh.z, xh.w);
-            mma_bf16(d[1], h0.z, h1.z, h0.w, h1.w, xl.z, xl.w);
-            mma_bf16(d[2], l0.z, l1.z, l0.w, l1.w, xh.z, xh.w);
-        };
+        float v0[4], v1[4];
         {
             uint4 xh[kWarpKB], xl[kWarpKB];
-#pragma unroll
-            for (int kb = 0; kb < kWarpKB; ++kb) {
-                xh[kb] = __ldcg(x0 + kb * 4);
-                xl[kb] = __ldcg(x0 + plane + kb * 4);
-            }
-#pragma unroll
-            for (int kb = 0; kb < kWarpKB; ++kb) product(kb, xh[kb], xl[kb], acc[0]);
+            load_x(xh, xl, x0, plane);
+            product(f, xh, xl, v0);
         }
         if (two) {
             uint4 xh[kWarpKB], xl[kWarpKB];
-#pragma unroll
-            for (int kb = 0; kb < kWarpKB; ++kb) {
-                xh[kb] = __ldcg(x1 + kb * 4);
-                xl[kb] = __ldcg(x1 + plane + kb * 4);
-            }
-#pragma unroll
-            for (int kb = 0; kb < kWarpKB; ++kb) product(kb, xh[kb], xl[kb], acc[1]);
+            load_x(xh, xl, x1, plane);
+            product(f, xh, xl, v1);
         }
-        // partial tiles of the four warps -> shared memory, [column][row]
-        float* mine = P[buf][qwarp];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            if (j && !two) break;
-            float v[4];
-#pragma unroll
-            for (int i = 0; i < 4; ++i) v[i] = acc[j][0][i] + (acc[j][1][i] + acc[j][2][i]);
-            float* o = mine + (8 * j + 2 * q) * kPStride + g;
-            o[0] = v[0];
-            o[kPStride] = v[1];
-            o[8] = v[2];
-            o[kPStride + 8] = v[3];
-        }
-        asm volatile("bar.sync %0, %1;" ::"r"(quad + 1), "r"(kQuadWarps * 32) : "memory");
+        store_partial(P[buf][qwarp], 0, lane, v0);
+        if (two) store_partial(P[buf][qwarp], 1, lane, v1);
+        quad_barrier(quad);
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             if (j && !two) break;
             const int at = ((qt >> 4) + 8 * j) * kPStride + r16;
-            const float sum = (P[buf][0][at] + P[buf][1][at]) + (P[buf][2][at] + P[buf][3][at]);
+            const float sum = sum_partials(P[buf], at);
             const uint32_t e = j ? eo1 : eo0;
             const size_t b = e & kSeqMask;
             const bool ok = n0 + (qt >> 4) + 8 * j < n;
@@ -316,13 +403,9 @@ __device__ __forceinline__ void run_phase(const LoopState& L, Fragments& f, cons
             if (PHASE == kPhaseA && rec) {
                 if (ok) __stcg(L.part + b * kGates + (row - kGates), v);
             } else if (PHASE == kPhaseA || PHASE == kPhaseB) {
-                // the four gates of a unit sit in four neighbouring lanes
-                const int gate = lane & 3, base = lane & ~3;
-                const float act = gate == 2 ? tanhf(v) : sigmoid_f(v);
-                const float gi = __shfl_sync(0xffffffffu, act, base), gf = __shfl_sync(0xffffffffu, act, base + 1);
-                const float gg = __shfl_sync(0xffffffffu, act, base + 2), go = __shfl_sync(0xffffffffu, act, base + 3);
-                const float cn = gf * c_old[j] + gi * gg;
-                const float hn = go * tanhf(cn);
+                float cn, hn;
+                cell(v, c_old[j], lane, cn, hn);
+                const int gate = lane & 3;
                 if (ok) {
                     constexpr int layer = PHASE == kPhaseB ? 1 : 0;
                     const int slot = (int)(e >> 30) ^ 1, unit = row >> 2;
@@ -342,7 +425,11 @@ __device__ __forceinline__ void run_phase(const LoopState& L, Fragments& f, cons
                     L.z[BH + b * kH + row] = lo;
                 }
             } else {
-                if (ok) __stcg(L.logits + b * kOutPad + row, v);
+                tile_stat(v, tile, row, lane, ok, L.stat + (set * s.n_seq + b) * kOutTiles, L.tail + (set * s.n_seq + b) * 16);
+                if (ok && s.trace && row < kJointOut) {
+                    const int nsteps = __ldcg(s.n_steps + b);
+                    if (nsteps < s.trace_cap) s.trace[(b * s.trace_cap + nsteps) * kJointOut + row] = v;
+                }
             }
         }
         buf ^= 1;  // the other buffer: its readers are behind the barrier above
@@ -351,51 +438,18 @@ __device__ __forceinline__ void run_phase(const LoopState& L, Fragments& f, cons
 
 // One warp per sequence: arg-max, confidence, record, commit, advance (src/model.rs:79-90,180-209), the joint input of
 // the next frame where the predictor output stays valid, and the lists of the next step.
-__device__ __forceinline__ void decide(const LoopState& L, uint32_t entry, int lane, uint32_t* next_live, uint32_t* next_upd, int* next_counts) {
+__device__ __forceinline__ void decide(const LoopState& L, uint32_t entry, int lane, size_t set, uint32_t* next_live, uint32_t* next_upd,
+                                       int* next_counts) {
     const DecodeState& s = L.s;
     const uint32_t b = entry & kSeqMask;
     const size_t BH = (size_t)s.n_seq * kH;
-    const float* lg = L.logits + (size_t)b * kOutPad;
-    constexpr int kPer = (kVocab + 31) / 32;
-    float v[kPer];
-#pragma unroll
-    for (int i = 0; i < kPer; ++i) v[i] = lane + 32 * i < kVocab ? __ldcg(lg + lane + 32 * i) : -INFINITY;
     const int frame = __ldcg(s.frame_idx + b), len = s.enc_len[b];
-    const int nsteps = __ldcg(s.n_steps + b), symbols = __ldcg(s.emitted + b);
-    float dl[kDurations];
-#pragma unroll
-    for (int i = 0; i < kDurations; ++i) dl[i] = __ldcg(lg + kVocab + i);
-    float best = -INFINITY;
-    int token = 0x7fffffff;
-#pragma unroll
-    for (int i = 0; i < kPer; ++i)
-        if (v[i] > best) { best = v[i]; token = lane + 32 * i; }  // ascending index per lane: first maximum kept
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-        const float ov = __shfl_xor_sync(0xffffffffu, best, o);
-        const int oi = __shfl_xor_sync(0xffffffffu, token, o);
-        if (ov > best || (ov == best && oi < token)) { best = ov; token = oi; }
-    }
-    if (token == 0x7fffffff) token = 0;  // not one comparable logit: the first entry, as a scan from entry 0 leaves it
-    float sum = 0.0f;
-#pragma unroll
-    for (int i = 0; i < kPer; ++i)
-        if (lane + 32 * i < kVocab) sum += expf(v[i] - best);
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-    int dur = 0;
-#pragma unroll
-    for (int i = 1; i < kDurations; ++i)
-        if (dl[i] > dl[0]) { dl[0] = dl[i]; dur = i; }
-    if (s.trace && nsteps < s.trace_cap) {
-        float* tr = s.trace + ((size_t)b * s.trace_cap + nsteps) * kJointOut;
-        for (int i = lane; i < kJointOut; i += 32) tr[i] = __ldcg(lg + i);
-    }
-    const bool emit = token != kVocab - 1;
-    int emitted = symbols + (emit ? 1 : 0);
+    const int nsteps = __ldcg(s.n_steps + b), n_tokens = __ldcg(s.n_tokens + b);
+    int symbols = __ldcg(s.emitted + b);
+    const Decision d = decide_tokens(L.stat + (set * s.n_seq + b) * kOutTiles, L.tail + (set * s.n_seq + b) * 16, lane);
+    const bool emit = d.token != kVocab - 1;
     int nf = frame;
-    if (dur > 0) { nf += dur; emitted = 0; }
-    else if (!emit || emitted >= kMaxSymbols) { nf += 1; emitted = 0; }
+    advance(emit, d.dur, nf, symbols);
     if (!emit && nf < len) {
         // the cached predictor output stays valid: joint input of the new frame
         const float4* en = reinterpret_cast<const float4*>(s.enc_proj + (size_t)(s.enc_off[b] + nf) * kJointDim);
@@ -416,21 +470,12 @@ __device__ __forceinline__ void decide(const LoopState& L, uint32_t entry, int l
         // committing the state that produced the token (src/model.rs:188-189) is the flip of the parity
         const uint32_t next = emit ? entry ^ (1u << 30) : entry;
         if (emit) {
-            const int n = __ldcg(s.n_tokens + b);
-            if (n < s.max_tokens) {
-                const size_t o = (size_t)b * s.max_tokens + n;
-                s.out_tokens[o] = (uint32_t)token;
-                s.out_frames[o] = frame;
-                s.out_durs[o] = dur;
-                s.out_conf[o] = 1.0f / sum;
-            } else {
-                atomicExch(s.overflow, 1);
-            }
-            s.n_tokens[b] = n + 1;
-            s.last_token[b] = token;
+            record(s, b, n_tokens, d, frame);
+            s.n_tokens[b] = n_tokens + 1;
+            s.last_token[b] = d.token;
         }
         s.frame_idx[b] = nf;
-        s.emitted[b] = emitted;
+        s.emitted[b] = symbols;
         s.n_steps[b] = nsteps + 1;
         if (nf < len) {
             // the order of a list does not matter: the columns of a product are independent
@@ -440,36 +485,45 @@ __device__ __forceinline__ void decide(const LoopState& L, uint32_t entry, int l
     }
 }
 
+// Grid-wide barrier over co-resident CTAs (cooperative launch).  The wait is bounded: when it runs out the kernel raises
+// *error and leaves; the other CTAs then run out of time too.
+struct GridBarrier {
+    unsigned* counter;
+    int* error;
+    int* gave_up;  // shared memory
+    unsigned target = 0;
+    __device__ __forceinline__ GridBarrier(const LoopState& L, int* flag) : counter(L.barrier), error(L.error), gave_up(flag) {
+        if (threadIdx.x == 0) *gave_up = 0;
+    }
+    __device__ __forceinline__ bool sync() {
+        target += gridDim.x;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(counter) : "memory");
+            unsigned seen;
+            const long long t0 = clock64();
+            while (true) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(counter) : "memory");
+                if (seen >= target) break;
+                if (clock64() - t0 > 4000000000LL) {
+                    atomicExch(error, 1);
+                    *gave_up = 1;
+                    break;
+                }
+            }
+        }
+        __syncthreads();
+        return *gave_up == 0;
+    }
+};
+
 __global__ void __launch_bounds__(kDecThreads, 1)
 tdt_decode_tc_kernel(const __grid_constant__ LoopState L, int max_steps) {
     __shared__ __align__(16) float P[kQuads][2][kQuadWarps][16 * kPStride];
     __shared__ int gave_up;
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = warp / kQuadWarps, qwarp = warp % kQuadWarps;
     const int n_seq = L.s.n_seq;
-    unsigned target = 0;
-    if (tid == 0) gave_up = 0;
-    // Grid-wide barrier over co-resident CTAs (cooperative launch).  The wait is bounded: when it runs out the kernel raises
-    // *error and leaves; the other CTAs then run out of time too.
-    auto grid_barrier = [&]() -> bool {
-        target += gridDim.x;
-        __syncthreads();
-        if (tid == 0) {
-            asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(L.barrier) : "memory");
-            unsigned seen;
-            const long long t0 = clock64();
-            while (true) {
-                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(L.barrier) : "memory");
-                if (seen >= target) break;
-                if (clock64() - t0 > 4000000000LL) {
-                    atomicExch(L.error, 1);
-                    gave_up = 1;
-                    break;
-                }
-            }
-        }
-        __syncthreads();
-        return gave_up == 0;
-    };
+    GridBarrier grid(L, &gave_up);
     Fragments f;
     f.tile = nullptr;
     auto fetch_ahead = [&](int phase, int n) {
@@ -484,24 +538,270 @@ tdt_decode_tc_kernel(const __grid_constant__ LoopState L, int max_steps) {
         if (n.y > 0) {
             run_phase<kPhaseA>(L, f, upd, n.y, quad, qwarp, lane, P[quad]);
             fetch_ahead(kPhaseB, n.y);
-            if (!grid_barrier()) return;
+            if (!grid.sync()) return;
             run_phase<kPhaseB>(L, f, upd, n.y, quad, qwarp, lane, P[quad]);
             fetch_ahead(kPhaseC, n.y);
-            if (!grid_barrier()) return;
+            if (!grid.sync()) return;
             run_phase<kPhaseC>(L, f, upd, n.y, quad, qwarp, lane, P[quad]);
             fetch_ahead(kPhaseD, n.x);
-            if (!grid_barrier()) return;
+            if (!grid.sync()) return;
         }
-        run_phase<kPhaseD>(L, f, live, n.x, quad, qwarp, lane, P[quad]);
+        run_phase<kPhaseD>(L, f, live, n.x, quad, qwarp, lane, P[quad], step & 1);
         // the counters of the step after the next were last read when this step's predecessor began
         if (blockIdx.x == 0 && tid == 0) __stcg(reinterpret_cast<int2*>(L.counts) + (step + 2) % 3, make_int2(0, 0));
-        if (!grid_barrier()) return;
+        if (!grid.sync()) return;
         uint32_t* next_live = L.live + (size_t)((step + 1) & 1) * n_seq;
         uint32_t* next_upd = L.upd + (size_t)((step + 1) & 1) * n_seq;
         int* next_counts = L.counts + 2 * ((step + 1) % 3);
         for (int i = warp * gridDim.x + blockIdx.x; i < n.x; i += gridDim.x * (kDecThreads / 32))
-            decide(L, __ldcg(live + i), lane, next_live, next_upd, next_counts);
-        if (!grid_barrier()) return;
+            decide(L, __ldcg(live + i), lane, step & 1, next_live, next_upd, next_counts);
+        if (!grid.sync()) return;
+    }
+}
+
+// ---------------------------------------------------------------- few sequences
+// At most sixteen sequences: column b of every product is sequence b, every tile belongs to one four-warp group for the
+// whole call, and every CTA takes the decisions itself (from the tiles' statistics, a kilobyte per sequence), so that a
+// step over a blank has one grid barrier and one that follows an emission has four.  Groups 0..319 keep the fragments of
+// phase A (the first 160 swap to phase B's and back while others work), 320..384 those of phase D, 385..424 phase C's.
+// The cells' states stay in the registers of the groups that own the units.  Whole call, 188 frames, this kernel / the
+// general one: 1 clip 0.82 / 1.37 ms, 16 clips 2.17 / 2.48 (estimated from 17); the sixteen columns of two MMAs are the line.
+constexpr int kSmallSeqs = 16;
+constexpr int kSmallGroups = 2 * kLstmTiles + kOutTiles + kPredTiles;  // 425
+constexpr int kZStride = kH + 32;  // bf16 per joint input row in shared memory: eight rows on distinct banks
+constexpr size_t kSmallSmem = sizeof(bf16) * 2 * kSmallSeqs * kZStride;
+
+__global__ void __launch_bounds__(kDecThreads, 1)
+tdt_decode_small_kernel(const __grid_constant__ LoopState L, int max_steps) {
+    extern __shared__ __align__(16) bf16 zs[];  // [plane][sequence][kZStride]
+    __shared__ __align__(16) float P[kQuads][kQuadWarps][16 * kPStride];
+    __shared__ int gave_up;
+    __shared__ int sh_frame[kSmallSeqs], sh_symbols[kSmallSeqs], sh_token[kSmallSeqs], sh_tokens[kSmallSeqs], sh_steps[kSmallSeqs],
+        sh_len[kSmallSeqs], sh_row[kSmallSeqs];
+    __shared__ Decision sh_dec[kSmallSeqs];
+    __shared__ unsigned sh_live, sh_upd, sh_par;
+    const DecodeState& s = L.s;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = warp / kQuadWarps, qwarp = warp % kQuadWarps;
+    const int n = s.n_seq;
+    const bool two = n > 8;
+    const size_t BH = (size_t)n * kH;
+    const int me = quad * gridDim.x + blockIdx.x;
+    const bool does_a = me < 2 * kLstmTiles, does_b = me < kLstmTiles;
+    const bool does_d = !does_a && me < 2 * kLstmTiles + kOutTiles;
+    const bool does_c = !does_a && !does_d && me < kSmallGroups;
+    bool fills_z = false;  // some group of this CTA does phase D
+    for (int k = 0; k < kQuads; ++k) {
+        const int m = k * gridDim.x + blockIdx.x;
+        fills_z |= m >= 2 * kLstmTiles && m < 2 * kLstmTiles + kOutTiles;
+    }
+    GridBarrier grid(L, &gave_up);
+    const uint4* tile_a = does_a ? tile_of(L.w, kPhaseA, me) : nullptr;
+    const uint4* tile_b = does_b ? tile_of(L.w, kPhaseB, me) : nullptr;
+    Fragments f;
+    f.tile = nullptr;
+    if (does_a) fetch_fragments(f, tile_a, qwarp, lane);
+    if (does_d) fetch_fragments(f, tile_of(L.w, kPhaseD, me - 2 * kLstmTiles), qwarp, lane);
+    if (does_c) fetch_fragments(f, tile_of(L.w, kPhaseC, me - 2 * kLstmTiles - kOutTiles), qwarp, lane);
+    if (warp == 0) {
+        const int len = lane < n ? s.enc_len[lane] : 0;
+        if (lane < n) {
+            sh_len[lane] = len;
+            sh_row[lane] = s.enc_off[lane];
+            sh_frame[lane] = sh_symbols[lane] = sh_tokens[lane] = sh_steps[lane] = 0;
+            sh_token[lane] = kVocab - 1;  // the blank (src/model.rs:123)
+        }
+        const unsigned live = __ballot_sync(0xffffffffu, len > 0);
+        if (lane == 0) { sh_live = sh_upd = live; sh_par = 0; }
+    }
+    __syncthreads();
+    const int g = lane >> 2, q = lane & 3, qt = qwarp * 32 + lane, r16 = qt & 15;
+    const int colx[2] = {min(g, n - 1), min(8 + g, n - 1)};              // columns of this lane's operands
+    const int col[2] = {min(qt >> 4, n - 1), min(8 + (qt >> 4), n - 1)};  // columns this thread finishes
+    const bool mine[2] = {(qt >> 4) < n, 8 + (qt >> 4) < n};
+    float c0[2] = {0.0f, 0.0f}, c0_new[2] = {0.0f, 0.0f}, c1[2] = {0.0f, 0.0f}, c1_new[2] = {0.0f, 0.0f};
+
+    // product of this group's tile with the hidden vectors of `layer` (new: the candidates) -> P, summed by the caller
+    auto hidden_product = [&](int layer, bool fresh, unsigned par) {
+        float v[4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+            if (j && !two) break;
+            const int slot = ((par >> colx[j]) & 1) ^ (fresh ? 1 : 0);
+            const bf16* row = L.h + (size_t)(slot * 2 + layer) * 2 * BH + (size_t)colx[j] * kH;
+            uint4 xh[kWarpKB], xl[kWarpKB];
+            load_x(xh, xl, reinterpret_cast<const uint4*>(row) + qwarp * kWarpKB * 4 + q, BH / 8);
+            product(f, xh, xl, v);
+            store_partial(P[quad][qwarp], j, lane, v);
+        }
+        quad_barrier(quad);
+    };
+    auto put_hidden = [&](int layer, int b, unsigned par, int unit, float hn) {
+        const int slot = ((par >> b) & 1) ^ 1;
+        bf16 hi, lo;
+        split2(hn, hi, lo);
+        bf16* ho = L.h + (size_t)(slot * 2 + layer) * 2 * BH + (size_t)b * kH + unit;
+        if ((lane & 3) == 1) ho[0] = hi;
+        else if ((lane & 3) == 2) ho[BH] = lo;
+    };
+
+    for (int step = 0; step < max_steps; ++step) {
+        const unsigned live = sh_live, upd = sh_upd, par = sh_par;
+        if (live == 0) break;
+        const size_t set = step & 1;
+        if (upd) {
+            // ---- A
+            if (does_a) {
+                const bool rec = me >= kLstmTiles;
+                const int row = me * 16 + r16;
+                float add[2] = {0.0f, 0.0f};
+                if (!rec) {
+                    add[0] = __ldg(L.w.token_gates + (size_t)sh_token[col[0]] * kGates + row);
+                    if (two) add[1] = __ldg(L.w.token_gates + (size_t)sh_token[col[1]] * kGates + row);
+                }
+                hidden_product(rec ? 1 : 0, false, par);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    if (j && !two) break;
+                    const float v = sum_partials(P[quad], ((qt >> 4) + 8 * j) * kPStride + r16) + add[j];
+                    const bool ok = mine[j] && ((upd >> col[j]) & 1);
+                    if (rec) {
+                        if (ok) __stcg(L.part + (size_t)col[j] * kGates + (row - kGates), v);
+                    } else {
+                        float cn, hn;
+                        cell(v, c0[j], lane, cn, hn);
+                        if (ok) {
+                            c0_new[j] = cn;
+                            put_hidden(0, col[j], par, row >> 2, hn);
+                        }
+                    }
+                }
+                if (does_b) fetch_fragments(f, tile_b, qwarp, lane);
+            }
+            if (!grid.sync()) return;
+            // ---- B
+            if (does_b) {
+                const int row = me * 16 + r16;
+                float add[2];
+                add[0] = __ldcg(L.part + (size_t)col[0] * kGates + row) + __ldg(L.w.b1 + row);
+                add[1] = two ? __ldcg(L.part + (size_t)col[1] * kGates + row) + __ldg(L.w.b1 + row) : 0.0f;
+                hidden_product(0, true, par);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    if (j && !two) break;
+                    const float v = sum_partials(P[quad], ((qt >> 4) + 8 * j) * kPStride + r16) + add[j];
+                    float cn, hn;
+                    cell(v, c1[j], lane, cn, hn);
+                    if (mine[j] && ((upd >> col[j]) & 1)) {
+                        c1_new[j] = cn;
+                        put_hidden(1, col[j], par, row >> 2, hn);
+                    }
+                }
+                fetch_fragments(f, tile_a, qwarp, lane);
+            }
+            if (!grid.sync()) return;
+            // ---- C
+            if (does_c) {
+                const int row = (me - 2 * kLstmTiles - kOutTiles) * 16 + r16;
+                const float bias = __ldg(L.b_pred + row);
+                hidden_product(1, true, par);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    if (j && !two) break;
+                    const float v = sum_partials(P[quad], ((qt >> 4) + 8 * j) * kPStride + r16) + bias;
+                    if (mine[j] && ((upd >> col[j]) & 1)) __stcg(s.pred + (size_t)col[j] * kJointDim + row, v);
+                }
+            }
+            if (!grid.sync()) return;
+        }
+        // ---- D: joint input of every live sequence into shared memory, then the product
+        if (fills_z) {
+            for (int i = tid; i < n * (kJointDim / 4); i += kDecThreads) {
+                const int b = i / (kJointDim / 4), c4 = i % (kJointDim / 4);
+                if (!((live >> b) & 1)) continue;
+                const float4 x = __ldg(reinterpret_cast<const float4*>(s.enc_proj + (size_t)(sh_row[b] + sh_frame[b]) * kJointDim) + c4);
+                const float4 p = __ldcg(reinterpret_cast<const float4*>(s.pred + (size_t)b * kJointDim) + c4);
+                const float zv[4] = {fmaxf(x.x + p.x, 0.0f), fmaxf(x.y + p.y, 0.0f), fmaxf(x.z + p.z, 0.0f), fmaxf(x.w + p.w, 0.0f)};
+                __align__(8) bf16 hi[4], lo[4];
+#pragma unroll
+                for (int e = 0; e < 4; ++e) split2(zv[e], hi[e], lo[e]);
+                *reinterpret_cast<uint2*>(zs + (size_t)b * kZStride + 4 * c4) = *reinterpret_cast<const uint2*>(hi);
+                *reinterpret_cast<uint2*>(zs + (size_t)(kSmallSeqs + b) * kZStride + 4 * c4) = *reinterpret_cast<const uint2*>(lo);
+            }
+            __syncthreads();
+            if (does_d) {
+                const int tile = me - 2 * kLstmTiles, row = tile * 16 + r16;
+                const float bias = __ldg(L.w.b_out + row);
+                float v[4];
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    if (j && !two) break;
+                    const uint4* x = reinterpret_cast<const uint4*>(zs + (size_t)colx[j] * kZStride) + qwarp * kWarpKB * 4 + q;
+                    uint4 xh[kWarpKB], xl[kWarpKB];
+#pragma unroll
+                    for (int kb = 0; kb < kWarpKB; ++kb) {
+                        xh[kb] = x[kb * 4];
+                        xl[kb] = x[kSmallSeqs * kZStride / 8 + kb * 4];
+                    }
+                    product(f, xh, xl, v);
+                    store_partial(P[quad][qwarp], j, lane, v);
+                }
+                quad_barrier(quad);
+#pragma unroll
+                for (int j = 0; j < 2; ++j) {
+                    if (j && !two) break;
+                    const float lv = sum_partials(P[quad], ((qt >> 4) + 8 * j) * kPStride + r16) + bias;
+                    const bool ok = mine[j] && ((live >> col[j]) & 1);
+                    const size_t b = col[j];
+                    tile_stat(lv, tile, row, lane, ok, L.stat + (set * n + b) * kOutTiles, L.tail + (set * n + b) * 16);
+                    if (ok && s.trace && row < kJointOut && sh_steps[b] < s.trace_cap)
+                        s.trace[(b * s.trace_cap + sh_steps[b]) * kJointOut + row] = lv;
+                }
+            }
+        }
+        if (!grid.sync()) return;
+        // ---- E, in every CTA
+        for (int b = warp; b < n; b += kDecThreads / 32) {
+            if (!((live >> b) & 1)) continue;
+            const Decision d = decide_tokens(L.stat + (set * n + b) * kOutTiles, L.tail + (set * n + b) * 16, lane);
+            if (lane == 0) sh_dec[b] = d;
+        }
+        __syncthreads();
+        if (warp == 0) {
+            bool alive = false, emit = false;
+            if (lane < n && ((live >> lane) & 1)) {
+                const Decision d = sh_dec[lane];
+                emit = d.token != kVocab - 1;
+                if (emit) {
+                    if (blockIdx.x == lane) record(s, lane, sh_tokens[lane], d, sh_frame[lane]);
+                    sh_tokens[lane] += 1;
+                    sh_token[lane] = d.token;
+                }
+                int frame = sh_frame[lane], symbols = sh_symbols[lane];
+                advance(emit, d.dur, frame, symbols);
+                sh_frame[lane] = frame;
+                sh_symbols[lane] = symbols;
+                sh_steps[lane] += 1;
+                alive = frame < sh_len[lane];
+            }
+            const unsigned la = __ballot_sync(0xffffffffu, alive), em = __ballot_sync(0xffffffffu, emit);
+            if (lane == 0) {
+                sh_live = la;
+                sh_upd = la & em;
+                sh_par = par ^ em;  // committing the state that produced the token (src/model.rs:188-189)
+            }
+        }
+        __syncthreads();
+        const unsigned emitted = par ^ sh_par;
+#pragma unroll
+        for (int j = 0; j < 2; ++j)
+            if ((emitted >> col[j]) & 1) {
+                c0[j] = c0_new[j];
+                c1[j] = c1_new[j];
+            }
+    }
+    if (blockIdx.x == 0 && tid < n) {
+        s.n_tokens[tid] = sh_tokens[tid];
+        s.n_steps[tid] = sh_steps[tid];
     }
 }
 
@@ -517,7 +817,7 @@ __global__ void dec_init_kernel(LoopState L) {
 constexpr size_t align256(size_t n) { return (n + 255) / 256 * 256; }
 
 struct ScratchLayout {
-    size_t h, c, z, part, logits, live, upd, counts, barrier, total;
+    size_t h, c, z, part, stat, tail, live, upd, counts, barrier, total;
     explicit ScratchLayout(int n_seq) {
         const size_t B = (size_t)n_seq;
         size_t at = 0;
@@ -529,7 +829,8 @@ struct ScratchLayout {
         barrier = take(sizeof(unsigned));
         z = take(2 * B * kH * sizeof(bf16));
         part = take(B * kGates * sizeof(float));
-        logits = take(B * kOutPad * sizeof(float));
+        stat = take(2 * B * kOutTiles * sizeof(float4));
+        tail = take(2 * B * 16 * sizeof(float));
         live = take(2 * B * sizeof(uint32_t));
         upd = take(2 * B * sizeof(uint32_t));
         total = at;
@@ -615,7 +916,8 @@ cudaError_t decode_tc_run(const DecodeWeights& w, const DecodeTcWeights& t, cons
     L.c = reinterpret_cast<float*>(base + lay.c);
     L.z = reinterpret_cast<bf16*>(base + lay.z);
     L.part = reinterpret_cast<float*>(base + lay.part);
-    L.logits = reinterpret_cast<float*>(base + lay.logits);
+    L.stat = reinterpret_cast<float4*>(base + lay.stat);
+    L.tail = reinterpret_cast<float*>(base + lay.tail);
     L.live = reinterpret_cast<uint32_t*>(base + lay.live);
     L.upd = reinterpret_cast<uint32_t*>(base + lay.upd);
     L.counts = reinterpret_cast<int*>(base + lay.counts);
@@ -623,8 +925,15 @@ cudaError_t decode_tc_run(const DecodeWeights& w, const DecodeTcWeights& t, cons
     L.error = d_error;
     cudaError_t e = cudaMemsetAsync(base, 0, lay.z, st);
     if (e != cudaSuccess) return e;
-    dec_init_kernel<<<std::min(32, (s.n_seq + 255) / 256), 256, 0, st>>>(L);
     void* args[] = {&L, &max_steps};
+    if (s.n_seq <= kSmallSeqs && sm_count * kQuads >= kSmallGroups) {
+        e = cudaFuncSetAttribute(tdt_decode_small_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmallSmem);
+        if (e != cudaSuccess) return e;
+        e = cudaLaunchCooperativeKernel((const void*)tdt_decode_small_kernel, dim3(sm_count), dim3(kDecThreads), args, kSmallSmem, st);
+        *launches += 1;
+        return e != cudaSuccess ? e : cudaGetLastError();
+    }
+    dec_init_kernel<<<std::min(32, (s.n_seq + 255) / 256), 256, 0, st>>>(L);
     e = cudaLaunchCooperativeKernel((const void*)tdt_decode_tc_kernel, dim3(sm_count), dim3(kDecThreads), args, 0, st);
     *launches += 2;
     return e != cudaSuccess ? e : cudaGetLastError();

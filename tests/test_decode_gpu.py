@@ -122,3 +122,25 @@ def test_many_sequences_span_several_gemm_tiles(ctx, weights, decode_path):
         alone = decode_gpu(ctx, [encs[i]], trace=False)[0]
         for k in ("tokens", "frames", "durations", "conf"):
             assert np.array_equal(alone[k], got[i][k])
+
+
+@pytest.mark.parametrize("n", [1, 8, 9, 16, 17, 33])
+def test_batch_sizes_around_the_kernel_lines(ctx, weights, n):
+    """One, two and more groups of eight columns, the largest batch of the few-sequences kernel and the smallest of the
+    general one: a clip gives the same numbers bit for bit in each, and equals its replay."""
+    rng = np.random.default_rng(n)
+    lens = [int(t) for t in rng.integers(0, 30, size=n - 1)] + [41]
+    encs = [rng.standard_normal((t, 1024)).astype(np.float32) for t in lens]
+    fill = [rng.standard_normal((5, 1024)).astype(np.float32) for _ in range(40)]
+    got = decode_gpu(ctx, encs)
+    larger = decode_gpu(ctx, fill + encs, trace=False)[len(fill):]
+    for g, h, t in zip(got, larger, lens):
+        if t == 0:
+            assert g["steps"] == h["steps"] == 0 and len(g["tokens"]) == 0
+            continue
+        rep = oracle.greedy_replay(g["logits"], time_steps=t)
+        assert rep["steps"] == g["steps"] == h["steps"]
+        for k in ("tokens", "frames", "durations", "conf"):
+            assert np.array_equal(g[k], h[k])
+            if k != "conf":
+                assert np.array_equal(rep[k], g[k])
