@@ -20,7 +20,7 @@
 // group keeps its tile's fragments in registers (80 per thread), over all sequences of the phase and, when a phase
 // repeats, over the iterations; the fragments of the phase to come are fetched before the barrier that starts it.
 // Against host-stepped tensor-memory GEMMs over a tripled K (eight kernels an iteration, all sequences in every product):
-// one clip of 188 frames 10.6 -> 1.37 ms, 280 clips of up to 187 frames 14.0 -> 6.7 ms for the whole call.
+// one clip of 188 frames 10.2 -> 0.82 ms, 280 clips 14.7 -> 6.5, 2236 clips 42.9 -> 37.2 ms for the whole call.
 //
 // fp32 operands go to the bf16 tensor cores as split sums: x = hi + lo with hi = bf16(x), lo = bf16(x - hi), and
 // x . w ~= hi.hi + hi.lo + lo.hi (the dropped term is below 2^-16 of |x||w|), each of the three in an fp32 accumulator of
@@ -137,8 +137,6 @@ __global__ void bias_kernel(const float* __restrict__ b1, float* __restrict__ b1
 }
 
 // ---------------------------------------------------------------- the loop
-__device__ __forceinline__ float sigmoid_f(float x) { return 1.0f / (1.0f + expf(-x)); }
-
 __device__ __forceinline__ void mma_bf16(float (&d)[4], uint32_t a0, uint32_t a1, uint32_t a2, uint32_t a3, uint32_t b0, uint32_t b1) {
     asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
                  : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
@@ -154,20 +152,21 @@ struct LoopState {
     // what the predictor computes from it; emitting a token flips the parity.  [slot][layer][plane hi / lo][n_seq][640]
     bf16* h;
     float* c;               // [slot][layer][n_seq][640]
-    bf16* z;                // [plane][n_seq][640] joint input
+    bf16* z;                // [n_seq][1280] joint input
     float* part;            // [n_seq][2560] recurrent half of layer 1's gates
     // Every tile of 16 joint outputs leaves {largest token logit, its index, sum of exp(logit - largest)} per sequence; the
     // last tile also leaves its logits (the blank and the durations).  Two sets, used in turn.
     float4* stat;           // [2][n_seq][65]
     float* tail;            // [2][n_seq][16]
-    // lists of the step (even / odd): sequences alive, sequences whose predictor must run; an entry is b | parity << 30
+    // lists of the step (even / odd): sequences alive, sequences whose predictor must run
     uint32_t *live, *upd;   // [2][n_seq]
     int* counts;            // [3][2]: alive, must run; three sets used in turn
     unsigned* barrier;
     int* error;
 };
 
-constexpr uint32_t kSeqMask = 0x3FFFFFFFu;
+constexpr uint32_t kSeqMask = 0x1FFFu, kTokenMask = 0x7FFu;  // a list entry: sequence | last token << 13 | parity << 30
+constexpr int kTokenShift = 13;
 
 enum { kPhaseA = 0, kPhaseB = 1, kPhaseC = 2, kPhaseD = 3 };
 
@@ -181,10 +180,6 @@ __device__ __forceinline__ const uint4* tile_of(const DecodeTcWeights& w, int ph
     const uint4* base = phase == kPhaseB ? w.ih1 : (phase == kPhaseC ? w.pred : w.out);
     return base + (size_t)t * kTileU4;
 }
-__device__ __forceinline__ constexpr int tiles_of(int phase) {
-    return phase == kPhaseA ? 2 * kLstmTiles : (phase == kPhaseB ? kLstmTiles : (phase == kPhaseC ? kPredTiles : kOutTiles));
-}
-
 __device__ __forceinline__ void fetch_fragments(Fragments& f, const uint4* tile, int qwarp, int lane) {
     if (f.tile == tile) return;
     f.tile = tile;
@@ -195,37 +190,54 @@ __device__ __forceinline__ void fetch_fragments(Fragments& f, const uint4* tile,
         for (int p = 0; p < 4; ++p) f.a[kb][p] = __ldg(src + (kb * 4 + p) * 32);
 }
 
-// A phase's work is (tiles x groups of 16 sequences), tile-major; each four-warp group takes a contiguous share of it, so
-// that it meets few tiles.
-struct Share {
-    int begin, end, groups;
+// Activations (hidden vectors, joint inputs) lie in global memory in the order in which a lane needs them: for every block of
+// 32 k and every q the eight hi values, then the eight lo values, 32 bytes that one load brings.  A warp's load then takes
+// eight whole 128-byte lines; with hi and lo in planes of their own it took half of sixteen (2236 clips 44.1 -> 37.2 ms
+// for the whole call, 280 clips 7.4 -> 6.4).
+constexpr int kRowElems = 2 * kH;  // bf16 per row
+__device__ __forceinline__ int elem_of(int k) { return (k >> 3) * 16 + (k & 7); }  // hi; the lo value is 8 further
+struct Pair {
+    uint4 hi, lo;
 };
-__device__ __forceinline__ Share share_of(int phase, int n, int quad) {
-    const int groups = (n + 15) >> 4;
-    const int64_t total = (int64_t)tiles_of(phase) * groups;
-    const int shares = gridDim.x * kQuads, me = quad * gridDim.x + blockIdx.x;
-    return {(int)(total * me / shares), (int)(total * (me + 1) / shares), groups};
+// Plain loads, which may hit in L1: the acquire of the grid barrier has discarded what L1 held before.
+__device__ __forceinline__ Pair load_pair(const bf16* p) {
+    Pair v;
+    asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+                 : "=r"(v.hi.x), "=r"(v.hi.y), "=r"(v.hi.z), "=r"(v.hi.w), "=r"(v.lo.x), "=r"(v.lo.y), "=r"(v.lo.z), "=r"(v.lo.w)
+                 : "l"(p)
+                 : "memory");
+    return v;
 }
-
-// Products of a warp's five k blocks: hi.hi, hi.lo and lo.hi into accumulators of their own.
-__device__ __forceinline__ void load_x(uint4 (&xh)[kWarpKB], uint4 (&xl)[kWarpKB], const uint4* x, size_t plane) {
+constexpr int kBlockElems = 4 * 16;  // bf16 from one block of 32 k to the next
+__device__ __forceinline__ void load_x(Pair (&x)[kWarpKB], const bf16* p) {
 #pragma unroll
-    for (int kb = 0; kb < kWarpKB; ++kb) {
-        xh[kb] = __ldcg(x + kb * 4);
-        xl[kb] = __ldcg(x + plane + kb * 4);
-    }
+    for (int kb = 0; kb < kWarpKB; ++kb) x[kb] = load_pair(p + kb * kBlockElems);
 }
-__device__ __forceinline__ void product(const Fragments& f, const uint4 (&xh)[kWarpKB], const uint4 (&xl)[kWarpKB], float (&v)[4]) {
+// Products of a warp's five k blocks: hi.hi, hi.lo and lo.hi into accumulators of their own.
+__device__ __forceinline__ void block_product(const uint4 (&a)[4], const Pair& x, float (&d)[3][4]) {
+    const uint4 xh = x.hi, xl = x.lo;
+    const uint4 h0 = a[0], h1 = a[1], l0 = a[2], l1 = a[3];
+    mma_bf16(d[0], h0.x, h1.x, h0.y, h1.y, xh.x, xh.y);
+    mma_bf16(d[1], h0.x, h1.x, h0.y, h1.y, xl.x, xl.y);
+    mma_bf16(d[2], l0.x, l1.x, l0.y, l1.y, xh.x, xh.y);
+    mma_bf16(d[0], h0.z, h1.z, h0.w, h1.w, xh.z, xh.w);
+    mma_bf16(d[1], h0.z, h1.z, h0.w, h1.w, xl.z, xl.w);
+    mma_bf16(d[2], l0.z, l1.z, l0.w, l1.w, xh.z, xh.w);
+}
+__device__ __forceinline__ void product(const Fragments& f, const Pair (&x)[kWarpKB], float (&v)[4]) {
+    float d[3][4] = {};
+#pragma unroll
+    for (int kb = 0; kb < kWarpKB; ++kb) block_product(f.a[kb], x[kb], d);
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = d[0][i] + (d[1][i] + d[2][i]);
+}
+// The same, refilling each block's registers with the next product's activations as soon as they have been used.
+__device__ __forceinline__ void product_refill(const Fragments& f, Pair (&x)[kWarpKB], float (&v)[4], const bf16* next, bool refill) {
     float d[3][4] = {};
 #pragma unroll
     for (int kb = 0; kb < kWarpKB; ++kb) {
-        const uint4 h0 = f.a[kb][0], h1 = f.a[kb][1], l0 = f.a[kb][2], l1 = f.a[kb][3];
-        mma_bf16(d[0], h0.x, h1.x, h0.y, h1.y, xh[kb].x, xh[kb].y);
-        mma_bf16(d[1], h0.x, h1.x, h0.y, h1.y, xl[kb].x, xl[kb].y);
-        mma_bf16(d[2], l0.x, l1.x, l0.y, l1.y, xh[kb].x, xh[kb].y);
-        mma_bf16(d[0], h0.z, h1.z, h0.w, h1.w, xh[kb].z, xh[kb].w);
-        mma_bf16(d[1], h0.z, h1.z, h0.w, h1.w, xl[kb].z, xl[kb].w);
-        mma_bf16(d[2], l0.z, l1.z, l0.w, l1.w, xh[kb].z, xh[kb].w);
+        block_product(f.a[kb], x[kb], d);
+        if (refill) x[kb] = load_pair(next + kb * kBlockElems);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) v[i] = d[0][i] + (d[1][i] + d[2][i]);
@@ -241,16 +253,30 @@ __device__ __forceinline__ void store_partial(float* mine, int j, int lane, cons
 __device__ __forceinline__ void quad_barrier(int quad) {
     asm volatile("bar.sync %0, %1;" ::"r"(quad + 1), "r"(kQuadWarps * 32) : "memory");
 }
-__device__ __forceinline__ float sum_partials(float (*P)[16 * kPStride], int at) { return (P[0][at] + P[1][at]) + (P[2][at] + P[3][at]); }
+template <int N>
+__device__ __forceinline__ float sum_partials(float (*P)[N], int at) { return (P[0][at] + P[1][at]) + (P[2][at] + P[3][at]); }
+
+// 1 / (1 + 2^(k x)) with the hardware's exponential and reciprocal (relative error about 2^-22 each): k = -log2(e) gives the
+// logistic function, k = -2 log2(e) gives (tanh(x) + 1) / 2.  A division, expf and tanhf in their place are some 250
+// dependent instructions per column, a third of a phase at 200 sequences.
+__device__ __forceinline__ float logistic_pow2(float x, float k) {
+    float e, r;
+    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * k));
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
+    return r;
+}
+constexpr float kNegLog2e = -1.4426950408889634f;
 
 // One LSTM unit: its four gates (i, f, g, o) sit in four neighbouring lanes, pre-activation v.
 __device__ __forceinline__ void cell(float v, float c_old, int lane, float& cn, float& hn) {
     const int base = lane & ~3;
-    const float act = (lane & 3) == 2 ? tanhf(v) : sigmoid_f(v);
+    const bool candidate = (lane & 3) == 2;  // a tanh; the other gates are logistic
+    const float r = logistic_pow2(v, candidate ? 2.0f * kNegLog2e : kNegLog2e);
+    const float act = candidate ? fmaf(2.0f, r, -1.0f) : r;
     const float gi = __shfl_sync(0xffffffffu, act, base), gf = __shfl_sync(0xffffffffu, act, base + 1);
     const float gg = __shfl_sync(0xffffffffu, act, base + 2), go = __shfl_sync(0xffffffffu, act, base + 3);
-    cn = gf * c_old + gi * gg;
-    hn = go * tanhf(cn);
+    cn = fmaf(gf, c_old, gi * gg);
+    hn = go * fmaf(2.0f, logistic_pow2(cn, 2.0f * kNegLog2e), -1.0f);
 }
 // The same sixteen lanes that hold a column of a joint output tile reduce it (row = lane % 16 of the tile).
 __device__ __forceinline__ void tile_stat(float v, int tile, int row, int lane, bool ok, float4* stat, float* tail) {
@@ -328,48 +354,81 @@ __device__ __forceinline__ void record(const DecodeState& s, uint32_t b, int n, 
     }
 }
 
+// ---------------------------------------------------------------- many sequences
+// A phase's work is (tiles x groups of 16 sequences), tile-major; each four-warp group takes a contiguous share of it, so that
+// it meets at most two or three tiles.  An item is a chain list entry -> activation rows -> products -> sum over the warps ->
+// epilogue of some 4000 cycles; the list entries are read one item ahead and every activation register is refilled for the
+// next product as soon as the current one has used it, so that the L2 latencies lie under the MMAs.  Sharing the rows of an
+// item among the three groups of a CTA (cp.async or bulk copies into shared memory) takes a third of the L2 traffic but was
+// slower, 5.9 and 7.6 ms against 5.0 for 280 clips: the groups then wait for one another.
+constexpr int kMaxSeqs = 8192;     // thirteen bits of a list entry
+
+__device__ __forceinline__ constexpr int tiles_of(int phase) {
+    return phase == kPhaseA ? 2 * kLstmTiles : (phase == kPhaseB ? kLstmTiles : (phase == kPhaseC ? kPredTiles : kOutTiles));
+}
+struct Share {
+    int begin, end, groups;
+};
+__device__ __forceinline__ Share share_of(int phase, int n, int quad) {
+    const int groups = (n + 15) >> 4;
+    const int64_t total = (int64_t)tiles_of(phase) * groups;
+    const int shares = gridDim.x * kQuads, me = quad * gridDim.x + blockIdx.x;
+    return {(int)(total * me / shares), (int)(total * (me + 1) / shares), groups};
+}
+
 template <int PHASE>
 __device__ __forceinline__ void run_phase(const LoopState& L, Fragments& f, const uint32_t* list, int n, int quad, int qwarp, int lane,
-                                          float (*P)[kQuadWarps][16 * kPStride], size_t set = 0) {
+                                          float (*sm)[kQuadWarps][16 * kPStride], size_t set = 0) {
     const DecodeState& s = L.s;
     const Share sh = share_of(PHASE, n, quad);
+    if (sh.begin >= sh.end) return;
     const size_t BH = (size_t)s.n_seq * kH;
-    const int g = lane >> 2, q = lane & 3, qt = qwarp * 32 + lane;
-    int buf = 0;
+    const int g = lane >> 2, q = lane & 3, qt = qwarp * 32 + lane, r16 = qt & 15;
+    // activation row of a list entry (this lane's part of it)
+    auto row_of = [&](uint32_t e, int tile) -> const bf16* {
+        const size_t b = e & kSeqMask;
+        const bf16* r;
+        if (PHASE == kPhaseD) {
+            r = L.z + b * kRowElems;
+        } else {
+            const int slot = (int)(e >> 30) ^ (PHASE == kPhaseA ? 0 : 1);
+            const int layer = PHASE == kPhaseA ? (tile >= kLstmTiles ? 1 : 0) : (PHASE == kPhaseB ? 0 : 1);
+            r = L.h + ((size_t)(slot * 2 + layer) * s.n_seq + b) * kRowElems;
+        }
+        return r + qwarp * kWarpKB * kBlockElems + q * 16;
+    };
+    int tile = sh.begin / sh.groups, n0 = (sh.begin - tile * sh.groups) * 16;
+    // a column beyond the list repeats the last one and is not stored
+    uint32_t e0 = __ldcg(list + min(n0 + g, n - 1)), e1 = __ldcg(list + min(n0 + 8 + g, n - 1));
+    fetch_fragments(f, tile_of(L.w, PHASE, tile), qwarp, lane);
+    Pair x[kWarpKB];
+    load_x(x, row_of(e0, tile));
     for (int item = sh.begin; item < sh.end; ++item) {
-        const int tile = item / sh.groups, n0 = (item - tile * sh.groups) * 16;
         const bool rec = PHASE == kPhaseA && tile >= kLstmTiles;  // the recurrent half of layer 1
-        const bool two = n - n0 > 8;
-        // rows of the activations: a column beyond the list repeats the last one and is not stored
-        const uint32_t e0 = __ldcg(list + min(n0 + g, n - 1));
-        const uint32_t e1 = __ldcg(list + min(n0 + 8 + g, n - 1));
-        const uint32_t eo0 = __ldcg(list + min(n0 + (qt >> 4), n - 1)), eo1 = __ldcg(list + min(n0 + 8 + (qt >> 4), n - 1));
-        auto row_of = [&](uint32_t e) -> const bf16* {
-            const size_t b = e & kSeqMask;
-            const int par = e >> 30;
-            if (PHASE == kPhaseD) return L.z + b * kH;
-            const int slot = PHASE == kPhaseA ? par : par ^ 1;
-            const int layer = PHASE == kPhaseA ? (rec ? 1 : 0) : (PHASE == kPhaseB ? 0 : 1);
-            return L.h + (size_t)(slot * 2 + layer) * 2 * BH + b * kH;
-        };
-        const uint4* x0 = reinterpret_cast<const uint4*>(row_of(e0)) + qwarp * kWarpKB * 4 + q;
-        const uint4* x1 = reinterpret_cast<const uint4*>(row_of(e1)) + qwarp * kWarpKB * 4 + q;
-        const size_t plane = BH / 8;  // uint4 from the hi to the lo plane
-        fetch_fragments(f, tile_of(L.w, PHASE, tile), qwarp, lane);
-        // what the epilogue adds, fetched while the product runs: thread qt finishes row qt % 16 of columns qt / 16 (+ 8)
-        const int row = tile * 16 + (qt & 15), r16 = qt & 15;
-        float add[2] = {0.0f, 0.0f}, c_old[2] = {0.0f, 0.0f};
+        const bool two = n - n0 > 8, more = item + 1 < sh.end;
+        const int row = tile * 16 + r16;
+        int next_tile = tile, next_n0 = n0 + 16;
+        if (next_n0 >= n) { next_n0 = 0; ++next_tile; }
+        uint32_t f0 = 0, f1 = 0;
+        if (more) {
+            f0 = __ldcg(list + min(next_n0 + g, n - 1));
+            f1 = __ldcg(list + min(next_n0 + 8 + g, n - 1));
+        }
+        // thread qt finishes row qt % 16 of columns qt / 16 (+ 8); what the epilogue adds is fetched under the product
+        uint32_t e[2];
+        e[0] = __shfl_sync(0xffffffffu, e0, 4 * (qt >> 4));
+        e[1] = __shfl_sync(0xffffffffu, e1, 4 * (qt >> 4));
+        float add[2], c_old[2];
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
-            const uint32_t e = j ? eo1 : eo0;
-            const size_t b = e & kSeqMask;
-            if (j && !two) continue;
+            const size_t b = e[j] & kSeqMask;
+            add[j] = c_old[j] = 0.0f;
             if (PHASE == kPhaseA && !rec) {
-                add[j] = __ldg(L.w.token_gates + (size_t)__ldcg(s.last_token + b) * kGates + row);
-                c_old[j] = __ldcg(L.c + (size_t)((e >> 30) * 2) * BH + b * kH + (row >> 2));
+                add[j] = __ldg(L.w.token_gates + (size_t)((e[j] >> kTokenShift) & kTokenMask) * kGates + row);
+                c_old[j] = __ldcg(L.c + (size_t)((e[j] >> 30) * 2) * BH + b * kH + (row >> 2));
             } else if (PHASE == kPhaseB) {
                 add[j] = __ldcg(L.part + b * kGates + row) + __ldg(L.w.b1 + row);
-                c_old[j] = __ldcg(L.c + (size_t)((e >> 30) * 2 + 1) * BH + b * kH + (row >> 2));
+                c_old[j] = __ldcg(L.c + (size_t)((e[j] >> 30) * 2 + 1) * BH + b * kH + (row >> 2));
             } else if (PHASE == kPhaseC) {
                 add[j] = __ldg(L.b_pred + row);
                 c_old[j] = __ldg(s.enc_proj + (size_t)(s.enc_off[b] + __ldcg(s.frame_idx + b)) * kJointDim + row);
@@ -378,61 +437,56 @@ __device__ __forceinline__ void run_phase(const LoopState& L, Fragments& f, cons
             }
         }
         float v0[4], v1[4];
-        {
-            uint4 xh[kWarpKB], xl[kWarpKB];
-            load_x(xh, xl, x0, plane);
-            product(f, xh, xl, v0);
-        }
-        if (two) {
-            uint4 xh[kWarpKB], xl[kWarpKB];
-            load_x(xh, xl, x1, plane);
-            product(f, xh, xl, v1);
-        }
-        store_partial(P[buf][qwarp], 0, lane, v0);
-        if (two) store_partial(P[buf][qwarp], 1, lane, v1);
-        quad_barrier(quad);
+        product_refill(f, x, v0, row_of(e1, tile), two);
+        if (two) product_refill(f, x, v1, row_of(f0, next_tile), more);
+        else if (more) load_x(x, row_of(f0, next_tile));
+        float (*P)[16 * kPStride] = sm[(item - sh.begin) & 1];
+        store_partial(P[qwarp], 0, lane, v0);
+        if (two) store_partial(P[qwarp], 1, lane, v1);
+        if (more && next_tile != tile) fetch_fragments(f, tile_of(L.w, PHASE, next_tile), qwarp, lane);
+        quad_barrier(quad);  // also: the other buffer's readers are done
 #pragma unroll
         for (int j = 0; j < 2; ++j) {
             if (j && !two) break;
-            const int at = ((qt >> 4) + 8 * j) * kPStride + r16;
-            const float sum = sum_partials(P[buf], at);
-            const uint32_t e = j ? eo1 : eo0;
-            const size_t b = e & kSeqMask;
+            const float val = sum_partials(P, ((qt >> 4) + 8 * j) * kPStride + r16) + add[j];
+            const size_t b = e[j] & kSeqMask;
             const bool ok = n0 + (qt >> 4) + 8 * j < n;
-            const float v = sum + add[j];
             if (PHASE == kPhaseA && rec) {
-                if (ok) __stcg(L.part + b * kGates + (row - kGates), v);
+                if (ok) __stcg(L.part + b * kGates + (row - kGates), val);
             } else if (PHASE == kPhaseA || PHASE == kPhaseB) {
                 float cn, hn;
-                cell(v, c_old[j], lane, cn, hn);
+                cell(val, c_old[j], lane, cn, hn);
                 const int gate = lane & 3;
                 if (ok) {
                     constexpr int layer = PHASE == kPhaseB ? 1 : 0;
-                    const int slot = (int)(e >> 30) ^ 1, unit = row >> 2;
+                    const int slot = (int)(e[j] >> 30) ^ 1, unit = row >> 2;
                     bf16 hi, lo;
                     split2(hn, hi, lo);
-                    bf16* ho = L.h + (size_t)(slot * 2 + layer) * 2 * BH + b * kH + unit;
+                    bf16* ho = L.h + ((size_t)(slot * 2 + layer) * s.n_seq + b) * kRowElems + elem_of(unit);
                     if (gate == 0) __stcg(L.c + (size_t)(slot * 2 + layer) * BH + b * kH + unit, cn);
                     else if (gate == 1) ho[0] = hi;
-                    else if (gate == 2) ho[BH] = lo;
+                    else if (gate == 2) ho[8] = lo;
                 }
             } else if (PHASE == kPhaseC) {
                 if (ok) {
                     bf16 hi, lo;
-                    split2(fmaxf(c_old[j] + v, 0.0f), hi, lo);
-                    __stcg(s.pred + b * kJointDim + row, v);
-                    L.z[b * kH + row] = hi;
-                    L.z[BH + b * kH + row] = lo;
+                    split2(fmaxf(c_old[j] + val, 0.0f), hi, lo);
+                    __stcg(s.pred + b * kJointDim + row, val);
+                    L.z[b * kRowElems + elem_of(row)] = hi;
+                    L.z[b * kRowElems + elem_of(row) + 8] = lo;
                 }
             } else {
-                tile_stat(v, tile, row, lane, ok, L.stat + (set * s.n_seq + b) * kOutTiles, L.tail + (set * s.n_seq + b) * 16);
+                tile_stat(val, tile, row, lane, ok, L.stat + (set * s.n_seq + b) * kOutTiles, L.tail + (set * s.n_seq + b) * 16);
                 if (ok && s.trace && row < kJointOut) {
                     const int nsteps = __ldcg(s.n_steps + b);
-                    if (nsteps < s.trace_cap) s.trace[(b * s.trace_cap + nsteps) * kJointOut + row] = v;
+                    if (nsteps < s.trace_cap) s.trace[(b * s.trace_cap + nsteps) * kJointOut + row] = val;
                 }
             }
         }
-        buf ^= 1;  // the other buffer: its readers are behind the barrier above
+        e0 = f0;
+        e1 = f1;
+        tile = next_tile;
+        n0 = next_n0;
     }
 }
 
@@ -442,7 +496,6 @@ __device__ __forceinline__ void decide(const LoopState& L, uint32_t entry, int l
                                        int* next_counts) {
     const DecodeState& s = L.s;
     const uint32_t b = entry & kSeqMask;
-    const size_t BH = (size_t)s.n_seq * kH;
     const int frame = __ldcg(s.frame_idx + b), len = s.enc_len[b];
     const int nsteps = __ldcg(s.n_steps + b), n_tokens = __ldcg(s.n_tokens + b);
     int symbols = __ldcg(s.emitted + b);
@@ -461,18 +514,17 @@ __device__ __forceinline__ void decide(const LoopState& L, uint32_t entry, int l
             __align__(8) bf16 hi[4], lo[4];
 #pragma unroll
             for (int e = 0; e < 4; ++e) split2(zv[e], hi[e], lo[e]);
-            uint2* zo = reinterpret_cast<uint2*>(L.z + (size_t)b * kH) + lane + 32 * i;
-            zo[0] = *reinterpret_cast<const uint2*>(hi);
-            zo[BH / 4] = *reinterpret_cast<const uint2*>(lo);
+            bf16* zo = L.z + (size_t)b * kRowElems + elem_of(4 * (lane + 32 * i));
+            *reinterpret_cast<uint2*>(zo) = *reinterpret_cast<const uint2*>(hi);
+            *reinterpret_cast<uint2*>(zo + 8) = *reinterpret_cast<const uint2*>(lo);
         }
     }
     if (lane == 0) {
         // committing the state that produced the token (src/model.rs:188-189) is the flip of the parity
-        const uint32_t next = emit ? entry ^ (1u << 30) : entry;
+        const uint32_t next = emit ? ((entry ^ (1u << 30)) & ~(kTokenMask << kTokenShift)) | ((uint32_t)d.token << kTokenShift) : entry;
         if (emit) {
             record(s, b, n_tokens, d, frame);
             s.n_tokens[b] = n_tokens + 1;
-            s.last_token[b] = d.token;
         }
         s.frame_idx[b] = nf;
         s.emitted[b] = symbols;
@@ -565,7 +617,7 @@ tdt_decode_tc_kernel(const __grid_constant__ LoopState L, int max_steps) {
 // step over a blank has one grid barrier and one that follows an emission has four.  Groups 0..319 keep the fragments of
 // phase A (the first 160 swap to phase B's and back while others work), 320..384 those of phase D, 385..424 phase C's.
 // The cells' states stay in the registers of the groups that own the units.  Whole call, 188 frames, this kernel / the
-// general one: 1 clip 0.82 / 1.37 ms, 16 clips 2.17 / 2.48 (estimated from 17); the sixteen columns of two MMAs are the line.
+// general one: 1 clip 0.82 / 1.37 ms; 16 clips here 2.01 ms, 17 clips there 2.39; the sixteen columns of two MMAs are the line.
 constexpr int kSmallSeqs = 16;
 constexpr int kSmallGroups = 2 * kLstmTiles + kOutTiles + kPredTiles;  // 425
 constexpr int kZStride = kH + 32;  // bf16 per joint input row in shared memory: eight rows on distinct banks
@@ -584,7 +636,6 @@ tdt_decode_small_kernel(const __grid_constant__ LoopState L, int max_steps) {
     const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = warp / kQuadWarps, qwarp = warp % kQuadWarps;
     const int n = s.n_seq;
     const bool two = n > 8;
-    const size_t BH = (size_t)n * kH;
     const int me = quad * gridDim.x + blockIdx.x;
     const bool does_a = me < 2 * kLstmTiles, does_b = me < kLstmTiles;
     const bool does_d = !does_a && me < 2 * kLstmTiles + kOutTiles;
@@ -627,10 +678,9 @@ tdt_decode_small_kernel(const __grid_constant__ LoopState L, int max_steps) {
         for (int j = 0; j < 2; ++j) {
             if (j && !two) break;
             const int slot = ((par >> colx[j]) & 1) ^ (fresh ? 1 : 0);
-            const bf16* row = L.h + (size_t)(slot * 2 + layer) * 2 * BH + (size_t)colx[j] * kH;
-            uint4 xh[kWarpKB], xl[kWarpKB];
-            load_x(xh, xl, reinterpret_cast<const uint4*>(row) + qwarp * kWarpKB * 4 + q, BH / 8);
-            product(f, xh, xl, v);
+            Pair x[kWarpKB];
+            load_x(x, L.h + ((size_t)(slot * 2 + layer) * n + colx[j]) * kRowElems + qwarp * kWarpKB * kBlockElems + q * 16);
+            product(f, x, v);
             store_partial(P[quad][qwarp], j, lane, v);
         }
         quad_barrier(quad);
@@ -639,9 +689,9 @@ tdt_decode_small_kernel(const __grid_constant__ LoopState L, int max_steps) {
         const int slot = ((par >> b) & 1) ^ 1;
         bf16 hi, lo;
         split2(hn, hi, lo);
-        bf16* ho = L.h + (size_t)(slot * 2 + layer) * 2 * BH + (size_t)b * kH + unit;
+        bf16* ho = L.h + ((size_t)(slot * 2 + layer) * n + b) * kRowElems + elem_of(unit);
         if ((lane & 3) == 1) ho[0] = hi;
-        else if ((lane & 3) == 2) ho[BH] = lo;
+        else if ((lane & 3) == 2) ho[8] = lo;
     };
 
     for (int step = 0; step < max_steps; ++step) {
@@ -735,14 +785,11 @@ tdt_decode_small_kernel(const __grid_constant__ LoopState L, int max_steps) {
 #pragma unroll
                 for (int j = 0; j < 2; ++j) {
                     if (j && !two) break;
-                    const uint4* x = reinterpret_cast<const uint4*>(zs + (size_t)colx[j] * kZStride) + qwarp * kWarpKB * 4 + q;
-                    uint4 xh[kWarpKB], xl[kWarpKB];
+                    const uint4* z = reinterpret_cast<const uint4*>(zs + (size_t)colx[j] * kZStride) + qwarp * kWarpKB * 4 + q;
+                    Pair x[kWarpKB];
 #pragma unroll
-                    for (int kb = 0; kb < kWarpKB; ++kb) {
-                        xh[kb] = x[kb * 4];
-                        xl[kb] = x[kSmallSeqs * kZStride / 8 + kb * 4];
-                    }
-                    product(f, xh, xl, v);
+                    for (int kb = 0; kb < kWarpKB; ++kb) x[kb] = {z[kb * 4], z[kSmallSeqs * kZStride / 8 + kb * 4]};
+                    product(f, x, v);
                     store_partial(P[quad][qwarp], j, lane, v);
                 }
                 quad_barrier(quad);
@@ -809,8 +856,9 @@ tdt_decode_small_kernel(const __grid_constant__ LoopState L, int max_steps) {
 __global__ void dec_init_kernel(LoopState L) {
     for (int b = blockIdx.x * 256 + threadIdx.x; b < L.s.n_seq; b += gridDim.x * 256)
         if (L.s.enc_len[b] > 0) {
-            L.live[atomicAdd(L.counts, 1)] = b;
-            L.upd[atomicAdd(L.counts + 1, 1)] = b;
+            const uint32_t entry = b | (uint32_t)(kVocab - 1) << kTokenShift;  // the blank comes first (src/model.rs:123)
+            L.live[atomicAdd(L.counts, 1)] = entry;
+            L.upd[atomicAdd(L.counts + 1, 1)] = entry;
         }
 }
 
@@ -906,6 +954,7 @@ cudaError_t decode_tc_enc_projection(const DecodeTcWeights& t, const float* d_en
 // Runs the greedy loop for s.n_seq sequences (the integer state is set up by the caller).
 cudaError_t decode_tc_run(const DecodeWeights& w, const DecodeTcWeights& t, const DecodeState& s, int max_steps,
                           int64_t enc_rows, void* scratch, int sm_count, int* d_error, int64_t* launches, cudaStream_t st) {
+    if (s.n_seq > kMaxSeqs) return cudaErrorInvalidValue;
     char* base = static_cast<char*>(scratch) + align256(sizeof(bf16) * (size_t)enc_rows * 3 * kDModel);
     const ScratchLayout lay(s.n_seq);
     LoopState L{};
