@@ -28,6 +28,7 @@
 #include <algorithm>
 
 #include "gemm.h"
+#include "launch.cuh"
 #include "tc_ptx.cuh"
 
 namespace sb {
@@ -46,7 +47,8 @@ constexpr int kSlabBytes = 32 * 128;  // per epilogue warp: 32 rows x 128 bytes
 // and its own half of the W rows, so a W tile crosses L2 -> SM once per 256 output rows instead of once per 128.
 template <int BN, int CTAS = 1>
 struct Cfg {
-    static constexpr int kStages = CTAS == 2 ? 6 : (BN == 256 ? 4 : 6);
+    static constexpr int kStages = BN <= 64 ? 8 : (CTAS == 2 ? 6 : (BN == 256 ? 4 : 6));
+    static constexpr int kHalves = BN >= 128 ? 2 : 1;  // column halves of a tile, each with four epilogue warps
     static constexpr int kABytes = kBM * kBKBytes;
     static constexpr int kBBytes = (BN / CTAS) * kBKBytes;
     static constexpr int kStageBytes = kABytes + kBBytes;
@@ -116,7 +118,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
         }
         for (int a = 0; a < 2; ++a) {
             mbar_init(tfull_bar(a), 1);
-            mbar_init(tempty_bar(a), kEpiWarps * CTAS);
+            mbar_init(tempty_bar(a), 4 * C::kHalves * CTAS);
         }
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -135,6 +137,8 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
     if constexpr (CTAS == 2) cluster_sync();  // the peer's barriers exist before anything arrives on them
     tc_fence_after();
     const uint32_t tmem_base = *tmem_slot;
+    pdl_trigger();  // not before the tensor memory is allocated: a successor's CTA on this SM must not take it first
+    pdl_wait();
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
@@ -222,11 +226,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
         const bool out_fp8 = ep.out_mode == kOutFp8;
         const bool glu = ep.act == kActGlu;
         // accumulator columns per slab: 128 bytes per output row in every mode
-        const int slab_cols = (out_fp8 || glu) ? 128 : (out_bf16 ? 64 : 32);
-        const int sw = lane & 7;
+        // (64 columns of a GLU tile narrower than 256 leave 64 bytes per row, with the 64-byte swizzle)
+        const bool narrow_glu = glu && BN / C::kHalves == 64;
+        const int slab_cols = (out_fp8 || glu) ? (narrow_glu ? 64 : 128) : (out_bf16 ? 64 : 32);
+        const int sw = narrow_glu ? (lane >> 1) & 3 : lane & 7;
+        const int slab_pitch = narrow_glu ? 64 : 128;
         uint32_t lt = 0;
         bool ok = true;
-        for (int t = tile0; t < num_tiles && ok; t += tile_step, ++lt) {
+        for (int t = half < C::kHalves ? tile0 : num_tiles; t < num_tiles && ok; t += tile_step, ++lt) {
             const int acc = lt & 1;
             const uint32_t acc_ph = (lt >> 1) & 1;
             const int m0 = (t / n_tiles) * kTileM + (int)rank * kBM, n0 = (t % n_tiles) * BN;
@@ -236,7 +243,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
             const float rs = (FP8 && ep.row_scale && row < ep.M) ? ep.row_scale[row] : 1.0f;
             const float out_inv = (out_fp8 && row < ep.M) ? 1.0f / ep.out_row_scale[row] : 1.0f;
             const uint32_t taddr = tmem_base + ((uint32_t)(quad * 32) << 16) + acc * BN;
-            const int cbeg = half * (BN / 2), cend = cbeg + BN / 2;
+            const int cbeg = half * (BN / C::kHalves), cend = cbeg + BN / C::kHalves;
 #pragma unroll 1
             for (int c = cbeg; c < cend; c += slab_cols) {
                 // the slab is free again once the previous TMA store has read it
@@ -291,7 +298,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
                             pk.z = *reinterpret_cast<uint32_t*>(&p2);
                             pk.w = *reinterpret_cast<uint32_t*>(&p3);
                             const int ch = 2 * sub + q;
-                            *reinterpret_cast<uint4*>(slab_ptr + lane * 128 + ((ch ^ sw) << 4)) = pk;
+                            *reinterpret_cast<uint4*>(slab_ptr + lane * slab_pitch + ((ch ^ sw) << 4)) = pk;
                         }
                     } else if (out_fp8) {
                         // 32 columns = 32 bytes = chunks 2*sub, 2*sub + 1 of this row
@@ -362,15 +369,15 @@ typedef CUresult (*EncodeTiledFn)(CUtensorMap*, CUtensorMapDataType, cuuint32_t,
 EncodeTiledFn g_encode = nullptr;
 int g_pair_tiles = 1;  // process-wide: 0 never, 1 where it pays (see gemm_launch), 2 every product large enough
 
-// 2-D row-major tensor [rows x cols] with a row pitch of `pitch_elems`; boxes of 128 bytes x box_rows, 128-byte swizzle.
+// 2-D row-major tensor [rows x cols] with a row pitch of `pitch_elems`; boxes of 128 (64) bytes x box_rows, swizzled over as many bytes.
 bool make_map(CUtensorMap* map, const void* ptr, int rows, int cols, int pitch_elems, CUtensorMapDataType dt,
-              int elem_bytes, int box_rows) {
+              int elem_bytes, int box_rows, int box_bytes = kBKBytes) {
     const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
     const cuuint64_t strides[1] = {(cuuint64_t)pitch_elems * elem_bytes};
-    const cuuint32_t box[2] = {(cuuint32_t)(kBKBytes / elem_bytes), (cuuint32_t)box_rows};
+    const cuuint32_t box[2] = {(cuuint32_t)(box_bytes / elem_bytes), (cuuint32_t)box_rows};
     const cuuint32_t estr[2] = {1, 1};
     CUresult r = g_encode(map, dt, 2, const_cast<void*>(ptr), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                          CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                          box_bytes == 64 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                           CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     return r == CUDA_SUCCESS;
 }
@@ -384,30 +391,13 @@ cudaError_t launch_t(const GemmArgs& g, int sm_count, int* d_error, cudaStream_t
     const CUtensorMapDataType out_dt = o8 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
                                           : (ob ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT32);
     if (!make_map(&ma, g.a, g.M, g.K, g.K, in_dt, eb, kBM) || !make_map(&mb, g.w, g.N, g.K, g.K, in_dt, eb, BN / CTAS) ||
-        !make_map(&mo, g.out, g.M, g.act == kActGlu ? g.N / 2 : g.N, g.ldo, out_dt, o8 ? 1 : (ob ? 2 : 4), 32))
+        !make_map(&mo, g.out, g.M, g.act == kActGlu ? g.N / 2 : g.N, g.ldo, out_dt, o8 ? 1 : (ob ? 2 : 4), 32,
+                  g.act == kActGlu && BN / Cfg<BN, CTAS>::kHalves == 64 ? 64 : kBKBytes))
         return cudaErrorInvalidValue;
     EpiParams ep{g.bias, g.row_scale, g.col_scale, g.out_row_scale, g.out, g.M, g.N, g.K, g.ldo, g.act, g.out_mode, g.alpha};
     const int tiles = ((g.M + kBM * CTAS - 1) / (kBM * CTAS)) * (g.N / BN);
-    if constexpr (CTAS == 2) {
-        const int pairs = std::min(tiles, sm_count / 2);
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = dim3(2 * pairs);
-        cfg.blockDim = dim3(kGemmThreads);
-        cfg.dynamicSmemBytes = Cfg<BN, CTAS>::kSmemBytes;
-        cfg.stream = stream;
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = 2;
-        attr[0].val.clusterDim.y = 1;
-        attr[0].val.clusterDim.z = 1;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        return cudaLaunchKernelEx(&cfg, gemm_kernel<BN, FP8, CTAS>, ma, mb, mo, ep, d_error);
-    } else {
-        const int grid = tiles < sm_count ? tiles : sm_count;
-        gemm_kernel<BN, FP8, CTAS><<<grid, kGemmThreads, Cfg<BN, CTAS>::kSmemBytes, stream>>>(ma, mb, mo, ep, d_error);
-        return cudaGetLastError();
-    }
+    const int grid = CTAS * std::min(tiles, sm_count / CTAS);
+    return launch_pdl(gemm_kernel<BN, FP8, CTAS>, dim3(grid), kGemmThreads, Cfg<BN, CTAS>::kSmemBytes, stream, CTAS, ma, mb, mo, ep, d_error);
 }
 
 }  // namespace
@@ -434,7 +424,7 @@ cudaError_t gemm_configure(const char** why) {
         return e;                                                                                           \
     }
     SB_SET(256, false, 1) SB_SET(128, false, 1) SB_SET(256, true, 1) SB_SET(128, true, 1)
-    SB_SET(256, false, 2) SB_SET(256, true, 2)
+    SB_SET(256, false, 2) SB_SET(256, true, 2) SB_SET(64, false, 1) SB_SET(32, false, 1)
 #undef SB_SET
     return cudaSuccess;
 }
@@ -448,15 +438,15 @@ cudaError_t gemm_launch(const GemmArgs& g, int sm_count, int* d_error, cudaStrea
         (reinterpret_cast<uintptr_t>(g.out) & 15) || (g.ldo & 7) || (reinterpret_cast<uintptr_t>(g.bias) & 15) ||
         (reinterpret_cast<uintptr_t>(g.col_scale) & 15))
         return cudaErrorInvalidValue;
-    // BN = 256 when it divides N and still leaves at least one tile per SM; else 128.
     const int m_tiles = (g.M + kBM - 1) / kBM;
     if (g.out_mode == kOutFp8 && (g.N % 256 != 0 || !g.out_row_scale || (g.ldo & 15))) return cudaErrorInvalidValue;
     if (g.act == kActGlu && (g.N % 256 != 0 || g.out_mode != kOutBf16)) return cudaErrorInvalidValue;
-    const bool wide = (g.N % 256 == 0) && (g.out_mode == kOutFp8 || g.act == kActGlu || m_tiles * (g.N / 256) >= sm_count);
     // Two CTAs per 256 x 256 tile when there is at least one such tile per pair of SMs.  Measured in the 8 h encoder
     // step against single-CTA tiles: residual-add products -15 % time (their fp32 epilogue leaves L2 little room
     // for operand traffic), K = 4096 products -9 %, QKV -6 %, the other K = 1024 products unchanged; the K = 256
     // sub-sampling products are 25 % slower (nothing to amortise), so short K stays on single-CTA tiles.
+    const bool wide_ok = g.N % 256 == 0;
+    const bool wide = wide_ok && (g.out_mode == kOutFp8 || g.act == kActGlu || m_tiles * (g.N / 256) >= sm_count);
     const bool pair = g_pair_tiles && wide && ((g.M + 2 * kBM - 1) / (2 * kBM)) * (g.N / 256) >= sm_count / 2 &&
                       (g_pair_tiles == 2 || g.K >= 512);
     if (g.fp8) {
@@ -464,7 +454,17 @@ cudaError_t gemm_launch(const GemmArgs& g, int sm_count, int* d_error, cudaStrea
         return wide ? launch_t<256, true, 1>(g, sm_count, d_error, stream) : launch_t<128, true, 1>(g, sm_count, d_error, stream);
     }
     if (pair) return launch_t<256, false, 2>(g, sm_count, d_error, stream);
-    return wide ? launch_t<256, false, 1>(g, sm_count, d_error, stream) : launch_t<128, false, 1>(g, sm_count, d_error, stream);
+    // Otherwise the narrowest tile with which the product is one wave.  An accumulator's chain of K / 16 dependent MMAs takes
+    // about 120 cycles a link however narrow the tile is (190 at 256 columns), so a wave costs nearly the same with all
+    // widths and what counts is that there is one, with a short epilogue.  Measured, us, at 32 / 64 / 128 / 256 columns:
+    // N = K = 1024, fp32 add: M = 188  8.4 / 9.3 / 10.2 / 12.5, M = 752  12.9 / 9.6 / 10.3 / 13.0, M = 4032  36 / 23.5 / 16.2 / 14.0;
+    // N = 1024, K = 4096: M = 188  21.7 / 22.6 / 23.6 / 31.6, M = 3008  108 / 58 / 42 / 31 (two waves of 128 against one of 256);
+    // N = 4096, K = 1024: M = 188  - / 9.8 / 10.5 / 13.1, M = 752  - / 19.0 / 15.5 / 13.6.  Bf16 rows want 64 columns a slab.
+    auto one_wave = [&](int bn) { return g.N % bn == 0 && m_tiles * (g.N / bn) <= sm_count; };
+    if (g.out_mode != kOutBf16 && one_wave(32)) return launch_t<32, false, 1>(g, sm_count, d_error, stream);
+    if (one_wave(64)) return launch_t<64, false, 1>(g, sm_count, d_error, stream);
+    if (one_wave(128) || !wide_ok) return launch_t<128, false, 1>(g, sm_count, d_error, stream);
+    return launch_t<256, false, 1>(g, sm_count, d_error, stream);
 }
 
 }  // namespace sb

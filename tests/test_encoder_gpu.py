@@ -204,3 +204,19 @@ def test_subsampling_tensor_core_kernel_against_cuda_core_kernel_and_oracle(ctx)
         assert np.linalg.norm(a - r) / np.linalg.norm(r) <= BF16_TOL, f.shape
         assert np.linalg.norm(b - r) / np.linalg.norm(r) <= BF16_TOL, f.shape
         assert np.linalg.norm(a - b) / np.linalg.norm(b) <= 1e-2, (f.shape, np.linalg.norm(a - b) / np.linalg.norm(b))
+
+
+@pytest.mark.parametrize("frames", [1, 9, 1017, 1025, 1033, 1501])
+def test_one_clip_equals_the_clip_in_a_batch(ctx, frames):
+    """A lone clip spreads its query blocks and channel blocks over CTAs and takes narrow product tiles; in a batch of 40 it
+    does not.  Encoder lengths 1, 2, 128, 129, 130 and 188: both sides of the line between one and two query blocks."""
+    import scriptrs_b200 as sb
+
+    w = eo.seeded_weights(eo.EncoderConfig(layers=1), seed=31, std=0.02, plain_norms=False)
+    sb.load_model(ctx, w, encoder_layers=1)
+    rng = np.random.default_rng(frames)
+    clip = rng.standard_normal((frames, 128)).astype(np.float32)
+    others = [rng.standard_normal((int(t), 128)).astype(np.float32) for t in rng.integers(1, 1502, 39)]
+    alone = run_gpu(ctx, [clip])[0]
+    batch = run_gpu(ctx, others[:20] + [clip] + others[20:])[20]
+    assert np.isfinite(alone).all() and np.array_equal(alone, batch)

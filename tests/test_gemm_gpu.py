@@ -114,3 +114,33 @@ def test_fp8_e4m3_with_row_and_channel_scales(ctx, tile_mode, M, N, K):
     assert torch.isfinite(out).all()
     err = (out - ref).norm() / ref.norm()
     assert err < 1e-5, float(err)   # same quantised operands on both sides: only the summation order differs
+
+
+@pytest.mark.parametrize("N,K,act,out_mode", [(1024, 1024, 0, 2), (1024, 256, 0, 1), (2048, 512, 0, 0), (3072, 256, 1, 0), (640, 192, 2, 1)])
+def test_a_row_does_not_depend_on_the_tile_width(ctx, N, K, act, out_mode):
+    """The number of rows chooses the tile (32, 64, 128 or 256 columns, one or two CTAs); every width adds an output's
+    products in the same order, so the leading rows of a large product equal those of a small one bit for bit.  The
+    small one is also checked against a float32 matmul."""
+    import scriptrs_b200 as sb
+
+    most = 4500
+    g = torch.Generator(device="cuda").manual_seed(N + K)
+    a = (torch.randn(most, K, device="cuda", generator=g) * 0.5).to(torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda", generator=g) * 0.05).to(torch.bfloat16)
+    bias = torch.randn(N, device="cuda", generator=g) * 0.1
+    dtype = torch.bfloat16 if out_mode == 0 else torch.float32
+
+    def run(m):
+        out = torch.full((m + 1, N), 3.0, device="cuda", dtype=dtype)
+        torch.cuda.synchronize()
+        sb.gemm(ctx, a.data_ptr(), w.data_ptr(), out.data_ptr(), m, N, K, d_bias=bias.data_ptr(), act=act, out_mode=out_mode)
+        ctx.synchronize()
+        assert (out[m] == 3.0).all()  # nothing beyond the last row
+        return out[:m]
+
+    whole = run(most)
+    for m in (1, 128, 129, 188, 376, 500, 752, 1184, 1504, 2400):
+        assert torch.equal(run(m), whole[:m]), m
+    acc = a[:376].float() @ w.float().t() + bias
+    ref = ref_epilogue(acc, None, act) + (3.0 if out_mode == 2 else 0.0)
+    assert (whole[:376].float() - ref).norm() / ref.norm() < (6e-3 if dtype == torch.bfloat16 else 1e-4)
