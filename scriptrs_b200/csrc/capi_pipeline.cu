@@ -91,8 +91,14 @@ int32_t transcribe_tasks(sb_ctx* c, const void* pcm_any, int64_t n_samples, cons
         SB_CUDA(c->pcm_stage.ensure(esz * (size_t)(hi - lo)));
         d_pcm = c->pcm_stage.p;
         // three pieces for large batches, two (1/8 + 7/8) for medium ones: at 280 tasks the single copy of 230 MB is
-        // 4-5 ms of exposed time, the second set of launches costs about 1 ms
-        if (ordered && n_tasks >= 512) n_pieces = 3;
+        // 4-5 ms of exposed time, the second set of launches costs about 1 ms.  A copy from pageable memory runs at a
+        // fifth of the rate: 7/8 of the samples then outlast 1/8 of the kernels, and three pieces pay from about 160
+        // tasks (pageable, two / three pieces: 121 tasks 40.5 / 41.4 ms, 163 54.0 / 52.6, 280 89.0 / 84.4, 466 150 / 138;
+        // pinned: 280 tasks 80.8 / 85.1).
+        cudaPointerAttributes attr{};
+        const bool pageable = cudaPointerGetAttributes(&attr, pcm) == cudaSuccess && attr.type == cudaMemoryTypeUnregistered;
+        (void)cudaGetLastError();
+        if (ordered && n_tasks >= (pageable ? 160 : 512)) n_pieces = 3;
         else if (ordered && n_tasks >= 64) n_pieces = 2;
         if (!c->copy_stream) SB_CUDA(cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking));
         while ((int)c->copy_events.size() < n_pieces + 1) {
@@ -693,65 +699,16 @@ int32_t run_vad_streamed(sb_ctx* c, const sb_vocab* vocab, const float* audio, i
     // largest pass 131072 / 65536 / 49152 / 32768 / 24576 windows: 456 / 425 / 422 / 433 / 472 ms: longer passes leave a
     // longer stretch to transcribe after the last recurrence, shorter ones make the pieces' kernels small)
     const int64_t pass_cap = std::min<int64_t>(c->vad_segment_windows, c->vad_stream_pass_windows);
-    std::vector<int64_t> cut{0};  // pass boundaries, in windows
-    for (int64_t w = 8192; cut.back() < n_win; w = std::min<int64_t>(2 * w, pass_cap))
-        cut.push_back(std::min(n_win, cut.back() + std::min<int64_t>(w, pass_cap)));
-    const int n_pass = (int)cut.size() - 1;
-    int64_t max_pass = 0;
-    for (int k = 0; k < n_pass; ++k) max_pass = std::max(max_pass, cut[k + 1] - cut[k]);
-    SB_CUDA(m.audio.ensure(sizeof(float) * (size_t)n_samples));
-    SB_CUDA(m.prob.ensure(sizeof(float) * (size_t)n_win));
-    m.host_prob.pinned_host = true;
-    SB_CUDA(m.host_prob.ensure(sizeof(float) * (size_t)n_win));
-    if (!c->vad_stream) {
-        int least = 0, greatest = 0;
-        SB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
-        SB_CUDA(cudaStreamCreateWithPriority(&c->vad_stream, cudaStreamNonBlocking, greatest));
-        SB_CUDA(cudaStreamCreateWithPriority(&c->vad_feed_stream, cudaStreamNonBlocking, greatest));
-    }
-    // events per pass: probabilities on the host | gate inputs ready | recurrence done; plus one that orders the passes
-    // after earlier work
-    while ((int)c->vad_events.size() < 3 * n_pass + 1) {
-        cudaEvent_t ev;
-        SB_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
-        c->vad_events.push_back(ev);
-    }
+    VadPasses passes;
+    int32_t s = passes.begin(c, audio, n_samples, 8192, pass_cap);
+    if (s != SB_OK) return s;
+    const int n_pass = passes.count();
+    const std::vector<int64_t>& cut = passes.cut;
     PieceRun run{c, m.audio.as<float>(), n_samples, lc.transcription};
     // room for the encoder frames of the whole recording windowed with overlap, plus a margin for short regions
-    int32_t s = run.begin(c->vad_rows_cap > 0 ? c->vad_rows_cap : (int64_t)(1.2 * (double)n_samples / 1280.0) + 16384);
+    s = run.begin(c->vad_rows_cap > 0 ? c->vad_rows_cap : (int64_t)(1.2 * (double)n_samples / 1280.0) + 16384);
     if (s != SB_OK) return s;
-    // Two streams feed the network: `fs` copies a pass's samples in and computes its gate inputs, `vs` runs the
-    // recurrences one after another; the gate inputs alternate between two buffers, so pass k + 1 is prepared while
-    // pass k recurs.
-    cudaStream_t vs = c->vad_stream, fs = c->vad_feed_stream;
-    cudaEvent_t* ev_host = c->vad_events.data();           // [k]: pass k's probabilities are in host memory
-    cudaEvent_t* ev_fed = c->vad_events.data() + n_pass;   // [k]: pass k's gate inputs are ready
-    cudaEvent_t* ev_rec = c->vad_events.data() + 2 * n_pass;  // [k]: pass k's recurrence has ended
-    cudaEvent_t ev_prior = c->vad_events[3 * n_pass];
-    // work of an earlier call on the context's stream may still read the buffers that the passes overwrite
-    SB_CUDA(cudaEventRecord(ev_prior, c->stream));
-    SB_CUDA(cudaStreamWaitEvent(vs, ev_prior, 0));
-    s = vad_begin(c, max_pass, vs, true);
-    if (s != SB_OK) return s;
-    SB_CUDA(cudaEventRecord(ev_prior, vs));
-    SB_CUDA(cudaStreamWaitEvent(fs, ev_prior, 0));
-    float* h_prob = m.host_prob.as<float>();
-    auto enqueue = [&](int k) -> int32_t {
-        const int64_t a = cut[k] * kVadWindow, b = std::min(n_samples, cut[k + 1] * kVadWindow);
-        const int n = (int)(cut[k + 1] - cut[k]);
-        if (k >= 2) SB_CUDA(cudaStreamWaitEvent(fs, ev_rec[k - 2], 0));  // the buffer's last reader
-        SB_CUDA(cudaMemcpyAsync(m.audio.as<float>() + a, audio + a, sizeof(float) * (size_t)(b - a), cudaMemcpyHostToDevice, fs));
-        int32_t r = vad_encode_pass(c, fs, m.audio.as<float>(), n_samples, cut[k], n, k & 1);
-        if (r != SB_OK) return r;
-        SB_CUDA(cudaEventRecord(ev_fed[k], fs));
-        SB_CUDA(cudaStreamWaitEvent(vs, ev_fed[k], 0));
-        r = vad_recur_pass(c, vs, cut[k], n, k & 1, m.prob.as<float>());
-        if (r != SB_OK) return r;
-        SB_CUDA(cudaEventRecord(ev_rec[k], vs));
-        SB_CUDA(cudaMemcpyAsync(h_prob + cut[k], m.prob.as<float>() + cut[k], sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost, vs));
-        SB_CUDA(cudaEventRecord(ev_host[k], vs));
-        return SB_OK;
-    };
+    float* h_prob = passes.host_prob();
     // The recurrence kernel holds one SM per CTA of its cluster for the length of a pass, and the GEMM and attention
     // kernels (one CTA per SM, each with a fixed share of the tiles, nearly all of the SM's shared memory) cannot sit
     // beside it: launched over all SMs, the CTAs that find their SM taken would run as a second wave.  So while passes
@@ -760,20 +717,19 @@ int32_t run_vad_streamed(sb_ctx* c, const sb_vocab* vocab, const float* audio, i
     c->sm_count = std::max(8, all_sms - c->vad_cluster);
     auto bail = [&](int32_t code) {
         const std::string msg = sb_last_error();
-        cudaStreamSynchronize(fs);
-        cudaStreamSynchronize(vs);
+        passes.drain();
         cudaStreamSynchronize(c->stream);
         c->sm_count = all_sms;
         return fail((sb_status)code, msg);
     };
-    s = enqueue(0);
+    s = passes.enqueue(0);
     if (s != SB_OK) return bail(s);
     SpeechRegionStream regions(n_samples, lc.vad.default_threshold, lc.segmentation);
     ExecutionPlan plan;
     size_t planned = 0;
     for (int k = 0; k < n_pass; ++k) {
-        if (k + 1 < n_pass && (s = enqueue(k + 1)) != SB_OK) return bail(s);
-        cudaError_t e = cudaEventSynchronize(ev_host[k]);
+        if (k + 1 < n_pass && (s = passes.enqueue(k + 1)) != SB_OK) return bail(s);
+        cudaError_t e = passes.wait(k);
         if (e != cudaSuccess) return bail(cuda_fail(e, "cudaEventSynchronize(vad pass)"));
         regions.push(h_prob + cut[k], cut[k + 1] - cut[k]);
         if (k + 1 == n_pass) regions.finish();
@@ -783,7 +739,7 @@ int32_t run_vad_streamed(sb_ctx* c, const sb_vocab* vocab, const float* audio, i
         if ((s = run.add(plan.tasks.data() + first_task, (int64_t)(plan.tasks.size() - first_task))) != SB_OK) return bail(s);
     }
     c->sm_count = all_sms;  // every pass has ended
-    if ((s = take_device_error(c, vs)) != SB_OK) return bail(s);  // a recurrence that gave up waiting
+    if ((s = take_device_error(c, c->vad_stream)) != SB_OK) return bail(s);  // a recurrence that gave up waiting
     sb_result* res = new sb_result();
     if (plan.tasks.empty()) {  // TranscriptionResult::empty (long_form.rs:206-208)
         res->r.duration_seconds = (double)n_samples / 16000.0;

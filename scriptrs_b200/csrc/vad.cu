@@ -669,4 +669,72 @@ int32_t vad_process_device(sb_ctx* c, const float* d_audio, int64_t n_samples, f
     return SB_OK;
 }
 
+float* VadPasses::host_prob() const { return c->vad->host_prob.as<float>(); }
+cudaError_t VadPasses::wait(int k) const { return cudaEventSynchronize(c->vad_events[k]); }
+void VadPasses::drain() const {
+    cudaStreamSynchronize(c->vad_feed_stream);
+    cudaStreamSynchronize(c->vad_stream);
+}
+
+int32_t VadPasses::begin(sb_ctx* ctx, const float* recording, int64_t n, int64_t first, int64_t cap) {
+    c = ctx;
+    audio = recording;
+    n_samples = n;
+    VadModel& m = *c->vad;
+    SB_CUDA(cudaSetDevice(c->device));
+    const int64_t n_win = (n + kVadWindow - 1) / kVadWindow;
+    cut.assign(1, 0);
+    int64_t max_pass = 0;
+    for (int64_t w = std::min(first, cap); cut.back() < n_win; w = std::min<int64_t>(2 * w, cap)) {
+        cut.push_back(std::min(n_win, cut.back() + w));
+        max_pass = std::max(max_pass, cut.back() - cut[cut.size() - 2]);
+    }
+    SB_CUDA(m.audio.ensure(sizeof(float) * (size_t)n));
+    SB_CUDA(m.prob.ensure(sizeof(float) * (size_t)n_win));
+    m.host_prob.pinned_host = true;
+    SB_CUDA(m.host_prob.ensure(sizeof(float) * (size_t)n_win));
+    if (!c->vad_stream) {
+        int least = 0, greatest = 0;
+        SB_CUDA(cudaDeviceGetStreamPriorityRange(&least, &greatest));
+        SB_CUDA(cudaStreamCreateWithPriority(&c->vad_stream, cudaStreamNonBlocking, greatest));
+        SB_CUDA(cudaStreamCreateWithPriority(&c->vad_feed_stream, cudaStreamNonBlocking, greatest));
+    }
+    // events per pass: probabilities on the host | gate inputs ready | recurrence done; plus one that orders the passes
+    // after earlier work
+    while ((int)c->vad_events.size() < 3 * count() + 1) {
+        cudaEvent_t ev;
+        SB_CUDA(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
+        c->vad_events.push_back(ev);
+    }
+    cudaEvent_t prior = c->vad_events[3 * count()];
+    // work of an earlier call on the context's stream may still read the buffers that the passes overwrite
+    SB_CUDA(cudaEventRecord(prior, c->stream));
+    SB_CUDA(cudaStreamWaitEvent(c->vad_stream, prior, 0));
+    const int32_t s = vad_begin(c, max_pass, c->vad_stream, true);
+    if (s != SB_OK) return s;
+    SB_CUDA(cudaEventRecord(prior, c->vad_stream));
+    SB_CUDA(cudaStreamWaitEvent(c->vad_feed_stream, prior, 0));
+    return SB_OK;
+}
+
+int32_t VadPasses::enqueue(int k) {
+    VadModel& m = *c->vad;
+    cudaStream_t vs = c->vad_stream, fs = c->vad_feed_stream;
+    cudaEvent_t *on_host = c->vad_events.data(), *fed = on_host + count(), *recurred = fed + count();
+    const int64_t a = cut[k] * kVadWindow, b = std::min(n_samples, cut[k + 1] * kVadWindow);
+    const int n = (int)(cut[k + 1] - cut[k]);
+    if (k >= 2) SB_CUDA(cudaStreamWaitEvent(fs, recurred[k - 2], 0));  // the buffer's last reader
+    SB_CUDA(cudaMemcpyAsync(m.audio.as<float>() + a, audio + a, sizeof(float) * (size_t)(b - a), cudaMemcpyHostToDevice, fs));
+    int32_t r = vad_encode_pass(c, fs, m.audio.as<float>(), n_samples, cut[k], n, k & 1);
+    if (r != SB_OK) return r;
+    SB_CUDA(cudaEventRecord(fed[k], fs));
+    SB_CUDA(cudaStreamWaitEvent(vs, fed[k], 0));
+    r = vad_recur_pass(c, vs, cut[k], n, k & 1, m.prob.as<float>());
+    if (r != SB_OK) return r;
+    SB_CUDA(cudaEventRecord(recurred[k], vs));
+    SB_CUDA(cudaMemcpyAsync(host_prob() + cut[k], m.prob.as<float>() + cut[k], sizeof(float) * (size_t)n, cudaMemcpyDeviceToHost, vs));
+    SB_CUDA(cudaEventRecord(on_host[k], vs));
+    return SB_OK;
+}
+
 }  // namespace sb

@@ -3,6 +3,8 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <vector>
+
 #include "context.h"
 
 namespace sb {
@@ -51,6 +53,20 @@ int32_t vad_process_device(sb_ctx* c, const float* d_audio, int64_t n_samples, f
 int32_t vad_begin(sb_ctx* c, int64_t max_pass_windows, cudaStream_t st, bool two_buffers);
 int32_t vad_encode_pass(sb_ctx* c, cudaStream_t st, const float* d_audio, int64_t n_samples, int64_t first, int n, int buf);
 int32_t vad_recur_pass(sb_ctx* c, cudaStream_t st, int64_t first, int n, int buf, float* d_prob);
+// A host recording through the network in passes on two high-priority streams: the copy and the gate inputs of pass k + 1
+// (feed) run beside the recurrence of pass k.  Pass sizes start at `first` windows and double up to `cap`.
+struct VadPasses {
+    sb_ctx* c = nullptr;
+    const float* audio = nullptr;
+    int64_t n_samples = 0;
+    std::vector<int64_t> cut;  // pass boundaries, in windows
+    int count() const { return (int)cut.size() - 1; }
+    float* host_prob() const;              // pinned; pass k's probabilities are there once wait(k) has returned
+    int32_t begin(sb_ctx* ctx, const float* recording, int64_t n, int64_t first, int64_t cap);
+    int32_t enqueue(int k);                // in order; the copy from pageable memory blocks the calling thread
+    cudaError_t wait(int k) const;
+    void drain() const;                    // both streams
+};
 // The device copy of the recording that the last sb_vad_process call on this context made (null if none).
 const float* vad_resident_audio(const sb_ctx* c);
 
