@@ -87,7 +87,7 @@ relpos_attention_tc_kernel(const __grid_constant__ CUtensorMap map_qkv, const __
     const uint32_t bar_qk = bar0, bar_q2 = bar0 + 8, bar_tab = bar0 + 16, bar_v = bar0 + 24;
     const uint32_t bar_sbd = bar0 + 32, bar_sac = bar0 + 40, bar_o = bar0 + 48;
 
-    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int tid = threadIdx.x, warp = warp_index(), lane = tid & 31;
     const int lg = warp & 3;   // tensor-memory lane group of this warp: rows 32 lg .. 32 lg + 31 of the block
     const int qd = warp >> 2;  // column quarter
     const int rl = 32 * lg + lane;
@@ -150,7 +150,7 @@ relpos_attention_tc_kernel(const __grid_constant__ CUtensorMap map_qkv, const __
     bool ok = true;
 
     int item = next_item(blockIdx.x);
-    if (item < n_items && tid == 0) {
+    if (item < n_items && warp == 0 && elect_one()) {
         load_q(item, first_block(item), bar_qk);
         load_v(item);
     }
@@ -167,7 +167,7 @@ relpos_attention_tc_kernel(const __grid_constant__ CUtensorMap map_qkv, const __
             const int i0 = qb * kAT;
             const bool last = qb == qb_end - 1;
             const int plo = max(0, (t - 1) - (i0 + kAT - 1));  // first local table row this block can reach
-            if (tid == 0) {
+            if (warp == 0 && elect_one()) {
                 mbar_expect_tx(bar_tab, 10 * kBoxBytes);
                 for (int kb = 0; kb < 2; ++kb)
                     for (int h = 0; h < 5; ++h)   // table rows plo .. plo + 319
@@ -233,7 +233,7 @@ relpos_attention_tc_kernel(const __grid_constant__ CUtensorMap map_qkv, const __
             tc_fence_before();
             if (!__syncthreads_and(mbar_wait(bar_tab, ph_tab, abort_flag))) { ok = false; break; }
             ph_tab ^= 1;
-            if (tid == 0) {
+            if (warp == 0 && elect_one()) {
                 tc_fence_after();
                 // S_bd first: its read-out (the shift pass) can start while S_ac is still being formed
 #pragma unroll
@@ -289,7 +289,7 @@ relpos_attention_tc_kernel(const __grid_constant__ CUtensorMap map_qkv, const __
             ph_sac ^= 1;
             tc_fence_after();
             // Q (and, after the last block, K) are no longer needed: fetch what comes next into their place
-            if (tid == 0) {
+            if (warp == 0 && elect_one()) {
                 if (!last) {
                     fence_proxy_async();
                     load_q(item, qb + 1, bar_q2);
@@ -361,7 +361,7 @@ relpos_attention_tc_kernel(const __grid_constant__ CUtensorMap map_qkv, const __
                 if (!__syncthreads_and(mbar_wait(bar_v, ph_v, abort_flag))) { ok = false; break; }
                 ph_v ^= 1;
             }
-            if (tid == 0) {
+            if (warp == 0 && elect_one()) {
                 tc_fence_after();
 #pragma unroll
                 for (int k = 0; k < kNK / 16; ++k) {
@@ -375,7 +375,7 @@ relpos_attention_tc_kernel(const __grid_constant__ CUtensorMap map_qkv, const __
             if (!__syncthreads_and(mbar_wait(bar_o, ph_o, abort_flag))) { ok = false; break; }
             ph_o ^= 1;
             tc_fence_after();
-            if (last && next < n_items && tid == 0) load_v(next);  // V was read by the tensor cores only
+            if (last && next < n_items && warp == 0 && elect_one()) load_v(next);  // V was read by the tensor cores only
             // O / sum -> bf16 -> staging rows -> coalesced global rows
             if (warp_live) {
                 const float inv = i < t ? 1.0f / ((part[rl] + part[kAT + rl]) + (part[2 * kAT + rl] + part3[rl])) : 0.0f;

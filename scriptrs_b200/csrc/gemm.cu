@@ -103,7 +103,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
         reinterpret_cast<uint32_t*>(base_ptr + S * C::kStageBytes + kEpiWarps * kSlabBytes + 8 * (2 * S + 4));
     volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const int warp = warp_index(), lane = threadIdx.x & 31;
     constexpr int kTileM = kBM * CTAS;
     const int m_tiles = (ep.M + kTileM - 1) / kTileM;
     const int n_tiles = ep.N / BN;
@@ -142,7 +142,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
 
     if (warp == 0) {
         // ------------------------------------------------------------ TMA producer
-        if (lane == 0) {
+        if (elect_one()) {
             uint32_t it = 0;
             bool ok = true;
             for (int t = tile0; t < num_tiles && ok; t += tile_step) {
@@ -174,7 +174,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
         }
     } else if (warp == 1) {
         // ------------------------------------------------------------ MMA issuer
-        if (lane == 0 && rank == 0) {
+        if (rank == 0 && elect_one()) {
             const uint32_t idesc = make_idesc<BN, FP8, CTAS>();
             uint32_t it = 0, lt = 0;
             bool ok = true;
@@ -247,7 +247,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
 #pragma unroll 1
             for (int c = cbeg; c < cend; c += slab_cols) {
                 // the slab is free again once the previous TMA store has read it
-                if (lane == 0) bulk_wait_read0();
+                if (elect_one()) bulk_wait_read0();
                 __syncwarp();
 #pragma unroll 1
                 for (int sub = 0; sub * 32 < slab_cols; ++sub) {
@@ -341,14 +341,14 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
                 }
                 fence_proxy_async();
                 __syncwarp();
-                if (lane == 0) {
+                if (elect_one()) {
                     if (ep.out_mode == kOutResidual) tma_reduce_add_2d(&tma_out, slab, n0 + c, m0 + quad * 32);
                     else tma_store_2d(&tma_out, slab, glu ? (n0 + c) >> 1 : n0 + c, m0 + quad * 32);
                     bulk_commit();
                 }
             }
         }
-        if (lane == 0) bulk_wait_all();
+        if (elect_one()) bulk_wait_all();
         __syncwarp();
     }
 
@@ -453,18 +453,38 @@ cudaError_t gemm_launch(const GemmArgs& g, int sm_count, int* d_error, cudaStrea
         if (pair) return launch_t<256, true, 2>(g, sm_count, d_error, stream);
         return wide ? launch_t<256, true, 1>(g, sm_count, d_error, stream) : launch_t<128, true, 1>(g, sm_count, d_error, stream);
     }
-    if (pair) return launch_t<256, false, 2>(g, sm_count, d_error, stream);
-    // Otherwise the narrowest tile with which the product is one wave.  An accumulator's chain of K / 16 dependent MMAs takes
-    // about 120 cycles a link however narrow the tile is (190 at 256 columns), so a wave costs nearly the same with all
-    // widths and what counts is that there is one, with a short epilogue.  Measured, us, at 32 / 64 / 128 / 256 columns:
-    // N = K = 1024, fp32 add: M = 188  8.4 / 9.3 / 10.2 / 12.5, M = 752  12.9 / 9.6 / 10.3 / 13.0, M = 4032  36 / 23.5 / 16.2 / 14.0;
-    // N = 1024, K = 4096: M = 188  21.7 / 22.6 / 23.6 / 31.6, M = 3008  108 / 58 / 42 / 31 (two waves of 128 against one of 256);
-    // N = 4096, K = 1024: M = 188  - / 9.8 / 10.5 / 13.1, M = 752  - / 19.0 / 15.5 / 13.6.  Bf16 rows want 64 columns a slab.
-    auto one_wave = [&](int bn) { return g.N % bn == 0 && m_tiles * (g.N / bn) <= sm_count; };
-    if (g.out_mode != kOutBf16 && one_wave(32)) return launch_t<32, false, 1>(g, sm_count, d_error, stream);
-    if (one_wave(64)) return launch_t<64, false, 1>(g, sm_count, d_error, stream);
-    if (one_wave(128) || !wide_ok) return launch_t<128, false, 1>(g, sm_count, d_error, stream);
-    return launch_t<256, false, 1>(g, sm_count, d_error, stream);
+    if (pair && g_pair_tiles == 2) return launch_t<256, false, 2>(g, sm_count, d_error, stream);
+    // The tile with the least waves x cost of a 64-wide step of K.  The costs (in 0.01 us) are those of products of one wave,
+    // where the ring's depth against the latency of the operands sets the pace: 0.15 us a step at 32 columns, 0.18 at 64,
+    // 0.22 at 128, 0.39 at 256 (the tensor core alone: 0.09, 0.10, 0.14, 0.27).  Measured, us, at 32 / 64 / 128 / 256 columns / pairs:
+    // N = K = 1024, fp32 add: M = 188  5.2 / 6.2 / 7.2 / 11.1 / 11.7, M = 752  7.6 / 6.5 / 7.6 / 11.7 / 12.5, M = 4032  19 / 14 / 12.3 / 12.5 / 13.4;
+    // N = 1024, K = 4096: M = 188  12.1 / 13.3 / 17.4 / 28.5 / 26.9, M = 1504  28.8 / 22.1 / 17.0 / 27.5 / 27.5, M = 4032  63 / 41 / 31 / 28.6 / 29.1;
+    // N = 4096, K = 1024: M = 188  - / 6.7 / 7.8 / 11.4 / 12.1, M = 1504  - / 18.7 / 15.1 / 17.6 / 18.3, M = 52000  - / 544 / 409 / 353 / 342.
+    // A bf16 row wants 64 columns for its slab.  Products with short K are bound by their epilogues: widest tile in one wave.
+    auto waves = [&](int bn) { return (int64_t)(m_tiles * (int64_t)(g.N / bn) + sm_count - 1) / sm_count; };
+    if (g.K < 512) {
+        if (wide) return launch_t<256, false, 1>(g, sm_count, d_error, stream);
+        for (int bn : {64, 128})
+            if (waves(bn) == 1) return bn == 64 ? launch_t<64, false, 1>(g, sm_count, d_error, stream) : launch_t<128, false, 1>(g, sm_count, d_error, stream);
+        return wide_ok ? launch_t<256, false, 1>(g, sm_count, d_error, stream) : launch_t<128, false, 1>(g, sm_count, d_error, stream);
+    }
+    int best = 0;
+    int64_t least = INT64_MAX;
+    auto offer = [&](int tile, int64_t cost) {
+        if (cost < least) { least = cost; best = tile; }
+    };
+    if (pair) offer(512, ((int64_t)((g.M + 2 * kBM - 1) / (2 * kBM)) * (g.N / 256) + sm_count / 2 - 1) / (sm_count / 2) * 39);
+    if (wide_ok) offer(256, waves(256) * 39);
+    offer(128, waves(128) * 22);
+    offer(64, waves(64) * 18);
+    if (g.out_mode != kOutBf16) offer(32, waves(32) * 15);
+    switch (best) {
+        case 512: return launch_t<256, false, 2>(g, sm_count, d_error, stream);
+        case 256: return launch_t<256, false, 1>(g, sm_count, d_error, stream);
+        case 128: return launch_t<128, false, 1>(g, sm_count, d_error, stream);
+        case 64: return launch_t<64, false, 1>(g, sm_count, d_error, stream);
+        default: return launch_t<32, false, 1>(g, sm_count, d_error, stream);
+    }
 }
 
 }  // namespace sb

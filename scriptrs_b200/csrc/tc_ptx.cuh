@@ -12,6 +12,17 @@ constexpr long long kWaitCycles = 4000000000LL;  // ~2 s at 1.9 GHz
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// True in one lane of the warp, always the same (all lanes call it).  tcgen05 and TMA instructions take their operands from uniform
+// registers: behind `if (lane == 0)` the compiler wraps every one of them in a loop over the active lanes (143 cycles an MMA,
+// measured), behind this it knows that there is one (64 cycles at 128 columns, 127 at 256: the tensor core's own rate).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t p;
+    asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+    return p != 0;
+}
+// Index of the warp, known to be the same in all its lanes.
+__device__ __forceinline__ int warp_index() { return __shfl_sync(0xffffffffu, (int)(threadIdx.x >> 5), 0); }
+
 __device__ __forceinline__ void mbar_init(uint32_t bar, uint32_t count) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(count));
 }
