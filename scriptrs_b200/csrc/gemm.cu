@@ -85,7 +85,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
             const __grid_constant__ CUtensorMap tma_out, EpiParams ep, int* __restrict__ error) {
     using C = Cfg<BN, CTAS>;
     // rank of this CTA in its pair (the pair's leader, rank 0, owns the barriers the MMAs wait on)
-    const uint32_t rank = CTAS == 2 ? cluster_ctarank() : 0u;
+    const uint32_t rank = CTAS == 2 ? __shfl_sync(0xffffffffu, cluster_ctarank(), 0) : 0u;
     constexpr int S = C::kStages;
     extern __shared__ unsigned char smem_dyn[];
     const uint32_t base = (smem_u32(smem_dyn) + 1023u) & ~1023u;
@@ -198,17 +198,16 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
                         else tc_mma<FP8>(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kt | k) ? 1u : 0u);
                     }
                     if constexpr (CTAS == 2) {
-                        // the ring slot is free in both CTAs once these MMAs have read it
-                        tc_commit_pair(mapa(empty_bar(s), 0));
-                        tc_commit_pair(mapa(empty_bar(s), 1));
+                        // the ring slot is free in both CTAs once these MMAs have read it (one commit for both barriers: two
+                        // of them took 5 % of a product of 52000 rows)
+                        tc_commit_both(empty_bar(s));
                     } else {
                         tc_commit(empty_bar(s));
                     }
                 }
                 if (ok) {
                     if constexpr (CTAS == 2) {
-                        tc_commit_pair(mapa(tfull_bar(acc), 0));
-                        tc_commit_pair(mapa(tfull_bar(acc), 1));
+                        tc_commit_both(tfull_bar(acc));
                     } else {
                         tc_commit(tfull_bar(acc));
                     }
@@ -456,10 +455,10 @@ cudaError_t gemm_launch(const GemmArgs& g, int sm_count, int* d_error, cudaStrea
     if (pair && g_pair_tiles == 2) return launch_t<256, false, 2>(g, sm_count, d_error, stream);
     // The tile with the least waves x cost of a 64-wide step of K.  The costs (in 0.01 us) are those of products of one wave,
     // where the ring's depth against the latency of the operands sets the pace: 0.15 us a step at 32 columns, 0.18 at 64,
-    // 0.22 at 128, 0.39 at 256 (the tensor core alone: 0.09, 0.10, 0.14, 0.27).  Measured, us, at 32 / 64 / 128 / 256 columns / pairs:
+    // 0.22 at 128, 0.39 at 256 (the tensor core alone: 0.09, 0.10, 0.14, 0.27), 0.37 for a pair's tile.  Measured, us, at 32 / 64 / 128 / 256 columns / pairs:
     // N = K = 1024, fp32 add: M = 188  5.2 / 6.2 / 7.2 / 11.1 / 11.7, M = 752  7.6 / 6.5 / 7.6 / 11.7 / 12.5, M = 4032  19 / 14 / 12.3 / 12.5 / 13.4;
     // N = 1024, K = 4096: M = 188  12.1 / 13.3 / 17.4 / 28.5 / 26.9, M = 1504  28.8 / 22.1 / 17.0 / 27.5 / 27.5, M = 4032  63 / 41 / 31 / 28.6 / 29.1;
-    // N = 4096, K = 1024: M = 188  - / 6.7 / 7.8 / 11.4 / 12.1, M = 1504  - / 18.7 / 15.1 / 17.6 / 18.3, M = 52000  - / 544 / 409 / 353 / 342.
+    // N = 4096, K = 1024: M = 188  - / 6.7 / 7.8 / 11.4 / 12.1, M = 1504  - / 18.7 / 15.1 / 17.6 / 18.3, M = 52000  - / 544 / 409 / 353 / 312.
     // A bf16 row wants 64 columns for its slab.  Products with short K are bound by their epilogues: widest tile in one wave.
     auto waves = [&](int bn) { return (int64_t)(m_tiles * (int64_t)(g.N / bn) + sm_count - 1) / sm_count; };
     if (g.K < 512) {
@@ -473,7 +472,7 @@ cudaError_t gemm_launch(const GemmArgs& g, int sm_count, int* d_error, cudaStrea
     auto offer = [&](int tile, int64_t cost) {
         if (cost < least) { least = cost; best = tile; }
     };
-    if (pair) offer(512, ((int64_t)((g.M + 2 * kBM - 1) / (2 * kBM)) * (g.N / 256) + sm_count / 2 - 1) / (sm_count / 2) * 39);
+    if (pair) offer(512, ((int64_t)((g.M + 2 * kBM - 1) / (2 * kBM)) * (g.N / 256) + sm_count / 2 - 1) / (sm_count / 2) * 37);
     if (wide_ok) offer(256, waves(256) * 39);
     offer(128, waves(128) * 22);
     offer(64, waves(64) * 18);
