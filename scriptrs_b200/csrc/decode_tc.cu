@@ -946,6 +946,7 @@ cudaError_t decode_tc_enc_projection(const DecodeTcWeights& t, const float* d_en
     g.out_mode = kOutF32;
     g.alpha = 1.0f;
     g.fp8 = false;
+    g.w_resident = true;
     const cudaError_t e = gemm_launch(g, sm_count, d_error, st);
     *launches += 2;
     return e != cudaSuccess ? e : cudaGetLastError();

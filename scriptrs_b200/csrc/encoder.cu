@@ -547,6 +547,7 @@ cudaError_t run_gemm(sb_ctx* c, const char* label, const void* a, const bf16* w,
     GemmArgs g{};
     g.a = a; g.w = w; g.bias = bias; g.out = out; g.M = M; g.N = N; g.K = K; g.ldo = act == kActGlu ? N / 2 : N; g.act = act;
     g.out_mode = mode; g.alpha = alpha; g.fp8 = false;
+    g.w_resident = true;
     c->launches += 1;
     c->prof.begin(label, c->stream);
     cudaError_t e = gemm_launch(g, c->sm_count, c->d_error, c->stream);
@@ -560,6 +561,7 @@ cudaError_t run_gemm_fp8(sb_ctx* c, const char* label, const uint8_t* a, const f
     GemmArgs g{};
     g.a = a; g.w = w; g.bias = bias; g.row_scale = a_scale; g.col_scale = w_scale; g.out = out; g.M = M; g.N = N; g.K = K;
     g.ldo = act == kActGlu ? N / 2 : N; g.act = act; g.out_mode = mode; g.alpha = alpha; g.fp8 = true; g.out_row_scale = out_row_scale;
+    g.w_resident = true;
     c->launches += 1;
     c->prof.begin(label, c->stream);
     cudaError_t e = gemm_launch(g, c->sm_count, c->d_error, c->stream);

@@ -29,6 +29,8 @@ struct GemmArgs {
     int out_mode;
     float alpha;
     bool fp8;
+    bool w_resident;         // w was complete before the kernel ahead of this one in the stream was launched (model weights):
+                             // it may be read before that kernel ends
 };
 
 // Process-wide switch for two-CTA 256 x 256 tiles: 0 never, 1 for the products that gain from them (default),
