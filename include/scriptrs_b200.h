@@ -298,10 +298,9 @@ int32_t sb_encode_device(sb_ctx* ctx, const float* d_feats, const int64_t* frame
 /* Batched ParakeetModel::greedy_decode (src/model.rs:64-95) with the state machine of
  * GreedyDecodeState (src/model.rs:98-214); the predictor (run_decoder, src/model.rs:344-364) and the
  * joint decision (run_joint, src/model.rs:366-384: token arg-max over 1025, duration arg-max over 5,
- * confidence = max softmax) run for the whole batch at once: by default every loop iteration is a short
- * sequence of tensor-core products and element-wise kernels replayed from a CUDA graph by the host, which
- * reads an "any sequence alive" word every few iterations; with the option "simt_decode" the whole loop
- * runs inside one persistent fp32 kernel.
+ * confidence = max softmax) run for the whole batch at once, the whole loop inside one persistent
+ * cooperative kernel: on the tensor cores with split-bf16 operands by default, in plain fp32 with the
+ * option "simt_decode".
  *   d_enc         device, packed [sum_i T'_i x 1024] f32, time-major per clip
  *   enc_offsets   host, n_clips + 1 prefix sums of T'_i
  *   max_tokens    capacity per clip of the four output arrays (host, [n_clips x max_tokens]);
