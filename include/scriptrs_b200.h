@@ -284,9 +284,11 @@ int64_t sb_weights_file_list(const char* path, char* buf, int64_t cap);
 int64_t sb_encoder_num_frames(int64_t feature_frames);
 
 /* Batched ParakeetModelInner::run_encoder (src/model.rs:327-342; CoreML contract src/coreml.rs:75-135).
- *   d_feats        device, packed [sum_i T_i x 128] f32 (the output of sb_frontend_device)
+ *   d_feats        device, packed [sum_i T_i x 128] f32 (the output of sb_frontend_device); any 4-byte boundary
+ *                  (fastest on a 16-byte one)
  *   frame_offsets  host, n_clips + 1 prefix sums of T_i
- *   d_out          device, packed [sum_i T'_i x 1024] f32, time-major per clip
+ *   d_out          device, packed [sum_i T'_i x 1024] f32, time-major per clip, on a 16-byte boundary (otherwise
+ *                  SB_INVALID_ARGUMENT)
  *   enc_offsets    host, n_clips + 1, written with the prefix sums of T'_i
  * Each clip is encoded with its exact length (no padding frames), which is what the reference's
  * blob does with `mel_length`.  T_i may not exceed 1501 (T' <= 188).  Asynchronous on the stream. */

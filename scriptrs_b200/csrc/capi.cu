@@ -538,6 +538,9 @@ int32_t sb_encode_device(sb_ctx* c, const float* d_feats, const int64_t* frame_o
     if (!c->model || !c->model->has_encoder) return fail(SB_MISSING_MODEL_ASSET, "no encoder weights loaded");
     if (n_clips <= 0) return fail(SB_EMPTY_AUDIO, "audio input was empty");
     if (n_clips > 65535) return fail(SB_INVALID_ARGUMENT, "at most 65535 clips per call");
+    // the closing LayerNorm writes 16 bytes a lane; a stack without blocks ends in a copy
+    if ((reinterpret_cast<uintptr_t>(d_feats) & 3) || (reinterpret_cast<uintptr_t>(d_out) & (c->model->layers > 0 ? 15 : 3)))
+        return fail(SB_INVALID_ARGUMENT, "the output buffer must be 16-byte aligned and the feature buffer aligned to its floats");
     for (int64_t i = 0; i < n_clips; ++i) {
         const int64_t t = frame_offsets[i + 1] - frame_offsets[i];
         if (t <= 0) return fail(SB_EMPTY_AUDIO, "clip without feature frames");

@@ -58,6 +58,9 @@ __device__ __forceinline__ uint32_t relu_pack(float a, float b) {
     return *reinterpret_cast<const uint32_t*>(&h);
 }
 
+// BYTES: size of one cp.async of the mel rows; 16 where the rows lie on 16-byte boundaries, else 4 (a caller's feature
+// buffer need only be aligned to its floats).
+template <int BYTES>
 __global__ void __launch_bounds__(256, 3)
 sub_conv0_dw1_tc_kernel(const float* __restrict__ feats, const int64_t* __restrict__ t0_off, const int* __restrict__ t1_off,
                         const int* __restrict__ t2_off, const uint2* __restrict__ w0_frag, const __half2* __restrict__ w1h,
@@ -76,14 +79,17 @@ sub_conv0_dw1_tc_kernel(const float* __restrict__ feats, const int64_t* __restri
 
     // mel rows 4 to0 - 3 .. 4 to0 + 4 TO - 1, zero outside the clip; the columns beside the 128 are zeroed once
     auto fetch = [&](int to0, int buf) {
-        for (int i = tid; i < kNX * (kMelBins / 4); i += 256) {
-            const int row = i / (kMelBins / 4), c4 = i % (kMelBins / 4);
+        constexpr int PF = BYTES / 4, PR = kMelBins / PF;  // floats per piece, pieces per row
+        for (int i = tid; i < kNX * PR; i += 256) {
+            const int row = i / PR, c = PF * (i % PR);
             const int r = 4 * to0 - 3 + row;
             const bool in = r >= 0 && r < T;
-            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.xs[buf][row][4 + 4 * c4]);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(feats + (base + (in ? r : 0)) * kMelBins + 4 * c4),
-                         "r"(in ? 16 : 0)
-                         : "memory");
+            const uint32_t dst = (uint32_t)__cvta_generic_to_shared(&sm.xs[buf][row][4 + c]);
+            const float* src = feats + (base + (in ? r : 0)) * kMelBins + c;
+            if constexpr (BYTES == 16)
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(in ? 16 : 0) : "memory");
+            else
+                asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(dst), "l"(src), "r"(in ? 4 : 0) : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
@@ -247,7 +253,9 @@ void subsample_build_dw(const float* w1_tap_major, const float* b1, uint32_t* ou
 }
 
 cudaError_t subsample_configure() {
-    return cudaFuncSetAttribute(sub_conv0_dw1_tc_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemLayout));
+    const cudaError_t e = cudaFuncSetAttribute(sub_conv0_dw1_tc_kernel<16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemLayout));
+    return e != cudaSuccess ? e
+                            : cudaFuncSetAttribute(sub_conv0_dw1_tc_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(SmemLayout));
 }
 
 cudaError_t subsample_conv0_dw1_launch(const float* feats, const int64_t* d_t0, const int* d_t1, const int* d_t2, int n_clips,
@@ -257,9 +265,10 @@ cudaError_t subsample_conv0_dw1_launch(const float* feats, const int64_t* d_t0, 
     const int pairs = (max_t2 + kTO - 1) / kTO;
     const int steps = (int64_t)pairs * n_clips >= (int64_t)4 * 12 * 148 ? 4 : 1;
     const dim3 grid((pairs + steps - 1) / steps, n_clips);
-    sub_conv0_dw1_tc_kernel<<<grid, 256, sizeof(SmemLayout), st>>>(feats, d_t0, d_t1, d_t2, static_cast<const uint2*>(w0_frag),
-                                                                  static_cast<const __half2*>(w1_pairs),
-                                                                  static_cast<__nv_bfloat16*>(out), steps);
+    if (reinterpret_cast<uintptr_t>(feats) & 3) return cudaErrorMisalignedAddress;
+    auto* kernel = reinterpret_cast<uintptr_t>(feats) & 15 ? sub_conv0_dw1_tc_kernel<4> : sub_conv0_dw1_tc_kernel<16>;
+    kernel<<<grid, 256, sizeof(SmemLayout), st>>>(feats, d_t0, d_t1, d_t2, static_cast<const uint2*>(w0_frag),
+                                                  static_cast<const __half2*>(w1_pairs), static_cast<__nv_bfloat16*>(out), steps);
     return cudaGetLastError();
 }
 

@@ -220,3 +220,31 @@ def test_one_clip_equals_the_clip_in_a_batch(ctx, frames):
     alone = run_gpu(ctx, [clip])[0]
     batch = run_gpu(ctx, others[:20] + [clip] + others[20:])[20]
     assert np.isfinite(alone).all() and np.array_equal(alone, batch)
+
+
+@pytest.mark.parametrize("offset", [1, 2, 3])
+def test_features_on_any_float_boundary(ctx, offset):
+    """A feature buffer that begins between two 16-byte boundaries gives what an aligned one gives, bit for bit (one clip and
+    a batch, first clip of odd length); an output buffer there is refused on the host, before any launch."""
+    import scriptrs_b200 as sb
+
+    w = eo.seeded_weights(eo.EncoderConfig(layers=1), seed=33, std=0.02, plain_norms=False)
+    sb.load_model(ctx, w, encoder_layers=1)
+    for frames in ([333], [77, 1501, 12, 1]):
+        rows = sum(frames)
+        room = torch.randn(rows * 128 + 4, device="cuda", generator=torch.Generator(device="cuda").manual_seed(offset + rows))
+        aligned = room[offset:offset + rows * 128].clone()
+        offs = np.concatenate([[0], np.cumsum(frames)]).astype(np.int64)
+        n_out = sum(sb.encoder_num_frames(t) for t in frames)
+        outs = []
+        for feats in (aligned, room[offset:]):
+            out = torch.full((n_out, 1024), float("nan"), device="cuda")
+            torch.cuda.synchronize()
+            sb.encode_device(ctx, feats.data_ptr(), offs, out.data_ptr())
+            ctx.synchronize()
+            outs.append(out)
+        assert torch.isfinite(outs[0]).all() and torch.equal(outs[0], outs[1])
+        launches = ctx.kernel_launches()
+        with pytest.raises(sb.ScriptrsError) as e:
+            sb.encode_device(ctx, aligned.data_ptr(), offs, outs[0].data_ptr() + 4 * offset)
+        assert e.value.status == 11 and ctx.kernel_launches() == launches
