@@ -48,7 +48,7 @@ constexpr int kSlabBytes = 32 * 128;  // per epilogue warp: 32 rows x 128 bytes
 template <int BN, int CTAS = 1>
 struct Cfg {
     static constexpr int kStages = BN <= 64 ? 8 : (CTAS == 2 ? 6 : (BN == 256 ? 4 : 6));
-    static constexpr int kHalves = BN >= 128 ? 2 : 1;  // column halves of a tile, each with four epilogue warps
+    static constexpr int kHalves = gemm_halves(BN);  // column halves of a tile, each with four epilogue warps
     static constexpr int kABytes = kBM * kBKBytes;
     static constexpr int kBBytes = (BN / CTAS) * kBKBytes;
     static constexpr int kStageBytes = kABytes + kBBytes;
@@ -251,7 +251,7 @@ gemm_kernel(const __grid_constant__ CUtensorMap tma_a, const __grid_constant__ C
         // accumulator columns per slab: 128 bytes per output row in every mode
         // (64 columns of a GLU tile narrower than 256 leave 64 bytes per row, with the 64-byte swizzle)
         const bool narrow_glu = glu && BN / C::kHalves == 64;
-        const int slab_cols = (out_fp8 || glu) ? (narrow_glu ? 64 : 128) : (out_bf16 ? 64 : 32);
+        const int slab_cols = gemm_slab_cols(ep.act, ep.out_mode, BN / C::kHalves);
         const int sw = narrow_glu ? (lane >> 1) & 3 : lane & 7;
         const int slab_pitch = narrow_glu ? 64 : 128;
         uint32_t lt = 0;
@@ -461,48 +461,15 @@ cudaError_t gemm_launch(const GemmArgs& g, int sm_count, int* d_error, cudaStrea
         (reinterpret_cast<uintptr_t>(g.out) & 15) || (g.ldo & 7) || (reinterpret_cast<uintptr_t>(g.bias) & 15) ||
         (reinterpret_cast<uintptr_t>(g.col_scale) & 15))
         return cudaErrorInvalidValue;
-    const int m_tiles = (g.M + kBM - 1) / kBM;
     if (g.out_mode == kOutFp8 && (g.N % 256 != 0 || !g.out_row_scale || (g.ldo & 15))) return cudaErrorInvalidValue;
     if (g.act == kActGlu && (g.N % 256 != 0 || g.out_mode != kOutBf16)) return cudaErrorInvalidValue;
-    // Two CTAs per 256 x 256 tile when there is at least one such tile per pair of SMs.  Measured in the 8 h encoder
-    // step against single-CTA tiles: residual-add products -15 % time (their fp32 epilogue leaves L2 little room
-    // for operand traffic), K = 4096 products -9 %, QKV -6 %, the other K = 1024 products unchanged; the K = 256
-    // sub-sampling products are 25 % slower (nothing to amortise), so short K stays on single-CTA tiles.
-    const bool wide_ok = g.N % 256 == 0;
-    const bool wide = wide_ok && (g.out_mode == kOutFp8 || g.act == kActGlu || m_tiles * (g.N / 256) >= sm_count);
-    const bool pair = g_pair_tiles && wide && ((g.M + 2 * kBM - 1) / (2 * kBM)) * (g.N / 256) >= sm_count / 2 &&
-                      (g_pair_tiles == 2 || g.K >= 512);
+    const GemmTile t = gemm_tile(g.M, g.N, g.K, g.fp8, g.act, g.out_mode, sm_count, g_pair_tiles);
     if (g.fp8) {
-        if (pair) return launch_t<256, true, 2>(g, sm_count, d_error, stream);
-        return wide ? launch_t<256, true, 1>(g, sm_count, d_error, stream) : launch_t<128, true, 1>(g, sm_count, d_error, stream);
+        if (t.ctas == 2) return launch_t<256, true, 2>(g, sm_count, d_error, stream);
+        return t.bn == 256 ? launch_t<256, true, 1>(g, sm_count, d_error, stream) : launch_t<128, true, 1>(g, sm_count, d_error, stream);
     }
-    if (pair && g_pair_tiles == 2) return launch_t<256, false, 2>(g, sm_count, d_error, stream);
-    // The tile with the least waves x cost of a 64-wide step of K.  The costs (in 0.01 us) are those of products of one wave,
-    // where the ring's depth against the latency of the operands sets the pace: 0.15 us a step at 32 columns, 0.18 at 64,
-    // 0.22 at 128, 0.39 at 256 (the tensor core alone: 0.09, 0.10, 0.14, 0.27), 0.37 for a pair's tile.  Measured, us, at 32 / 64 / 128 / 256 columns / pairs:
-    // N = K = 1024, fp32 add: M = 188  5.2 / 6.2 / 7.2 / 11.1 / 11.7, M = 752  7.6 / 6.5 / 7.6 / 11.7 / 12.5, M = 4032  19 / 14 / 12.3 / 12.5 / 13.4;
-    // N = 1024, K = 4096: M = 188  12.1 / 13.3 / 17.4 / 28.5 / 26.9, M = 1504  28.8 / 22.1 / 17.0 / 27.5 / 27.5, M = 4032  63 / 41 / 31 / 28.6 / 29.1;
-    // N = 4096, K = 1024: M = 188  - / 6.7 / 7.8 / 11.4 / 12.1, M = 1504  - / 18.7 / 15.1 / 17.6 / 18.3, M = 52000  - / 544 / 409 / 353 / 312.
-    // A bf16 row wants 64 columns for its slab.  Products with short K are bound by their epilogues: widest tile in one wave.
-    auto waves = [&](int bn) { return (int64_t)(m_tiles * (int64_t)(g.N / bn) + sm_count - 1) / sm_count; };
-    if (g.K < 512) {
-        if (wide) return launch_t<256, false, 1>(g, sm_count, d_error, stream);
-        for (int bn : {64, 128})
-            if (waves(bn) == 1) return bn == 64 ? launch_t<64, false, 1>(g, sm_count, d_error, stream) : launch_t<128, false, 1>(g, sm_count, d_error, stream);
-        return wide_ok ? launch_t<256, false, 1>(g, sm_count, d_error, stream) : launch_t<128, false, 1>(g, sm_count, d_error, stream);
-    }
-    int best = 0;
-    int64_t least = INT64_MAX;
-    auto offer = [&](int tile, int64_t cost) {
-        if (cost < least) { least = cost; best = tile; }
-    };
-    if (pair) offer(512, ((int64_t)((g.M + 2 * kBM - 1) / (2 * kBM)) * (g.N / 256) + sm_count / 2 - 1) / (sm_count / 2) * 37);
-    if (wide_ok) offer(256, waves(256) * 39);
-    offer(128, waves(128) * 22);
-    offer(64, waves(64) * 18);
-    if (g.out_mode != kOutBf16) offer(32, waves(32) * 15);
-    switch (best) {
-        case 512: return launch_t<256, false, 2>(g, sm_count, d_error, stream);
+    if (t.ctas == 2) return launch_t<256, false, 2>(g, sm_count, d_error, stream);
+    switch (t.bn) {
         case 256: return launch_t<256, false, 1>(g, sm_count, d_error, stream);
         case 128: return launch_t<128, false, 1>(g, sm_count, d_error, stream);
         case 64: return launch_t<64, false, 1>(g, sm_count, d_error, stream);

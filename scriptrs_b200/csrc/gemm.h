@@ -3,17 +3,9 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
-namespace sb {
+#include "gemm_tile.h"
 
-// kActGlu: the N accumulator columns are groups of 32 = 16 values followed by their 16 gates; the output has N / 2
-// columns, out[16 g + i] = v[32 g + i] * sigmoid(v[32 g + 16 + i]) (bf16 output, N % 256 == 0).
-enum GemmAct : int { kActNone = 0, kActSilu = 1, kActRelu = 2, kActGlu = 3 };
-enum GemmOut : int {
-    kOutBf16 = 0,      // out[M x N] bf16 = act(acc * scales + bias)
-    kOutF32 = 1,       // out[M x N] f32  = act(acc * scales + bias) * alpha
-    kOutResidual = 2,  // out[M x N] f32 += alpha * act(acc * scales + bias)
-    kOutFp8 = 3,       // out[M x N] e4m3 = act(acc * scales + bias) / out_row_scale[m]   (N % 256 == 0)
-};
+namespace sb {
 
 struct GemmArgs {
     const void* a;           // [M x K] row-major, bf16 (or e4m3 when fp8)
