@@ -256,28 +256,22 @@ __device__ __forceinline__ void quad_barrier(int quad) {
 template <int N>
 __device__ __forceinline__ float sum_partials(float (*P)[N], int at) { return (P[0][at] + P[1][at]) + (P[2][at] + P[3][at]); }
 
-// 1 / (1 + 2^(k x)) with the hardware's exponential and reciprocal (relative error about 2^-22 each): k = -log2(e) gives the
-// logistic function, k = -2 log2(e) gives (tanh(x) + 1) / 2.  A division, expf and tanhf in their place are some 250
-// dependent instructions per column, a third of a phase at 200 sequences.
-__device__ __forceinline__ float logistic_pow2(float x, float k) {
-    float e, r;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(e) : "f"(x * k));
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(1.0f + e));
-    return r;
-}
-constexpr float kNegLog2e = -1.4426950408889634f;
+__device__ __forceinline__ float logistic(float x) { return 1.0f / (1.0f + expf(-x)); }
 
-// One LSTM unit: its four gates (i, f, g, o) sit in four neighbouring lanes, pre-activation v.
-__device__ __forceinline__ void cell(float v, float c_old, int lane, float& cn, float& hn) {
-    const int base = lane & ~3;
-    const bool candidate = (lane & 3) == 2;  // a tanh; the other gates are logistic
-    const float r = logistic_pow2(v, candidate ? 2.0f * kNegLog2e : kNegLog2e);
-    const float act = candidate ? fmaf(2.0f, r, -1.0f) : r;
-    const float gi = __shfl_sync(0xffffffffu, act, base), gf = __shfl_sync(0xffffffffu, act, base + 1);
-    const float gg = __shfl_sync(0xffffffffu, act, base + 2), go = __shfl_sync(0xffffffffu, act, base + 3);
-    cn = fmaf(gf, c_old, gi * gg);
-    hn = go * fmaf(2.0f, logistic_pow2(cn, 2.0f * kNegLog2e), -1.0f);
+// One LSTM unit from its four gate pre-activations (i, f, g, o), in one thread: 64 of a group's 128 threads take the 4 units x
+// 16 columns of a tile.  With a gate per lane, logistic function and hyperbolic tangent in neighbouring lanes, every warp went
+// through both, and through the cell's own tangent four times over.
+__device__ __forceinline__ void cell(float4 v, float c_old, float& cn, float& hn) {
+    cn = fmaf(logistic(v.y), c_old, logistic(v.x) * tanhf(v.z));
+    hn = logistic(v.w) * tanhf(cn);
 }
+template <int N>
+__device__ __forceinline__ float4 sum_partials4(const float (*P)[N], int at) {
+    const float4 a = *reinterpret_cast<const float4*>(&P[0][at]), b = *reinterpret_cast<const float4*>(&P[1][at]);
+    const float4 c = *reinterpret_cast<const float4*>(&P[2][at]), d = *reinterpret_cast<const float4*>(&P[3][at]);
+    return make_float4((a.x + b.x) + (c.x + d.x), (a.y + b.y) + (c.y + d.y), (a.z + b.z) + (c.z + d.z), (a.w + b.w) + (c.w + d.w));
+}
+__device__ __forceinline__ float4 add4(float4 a, float4 b) { return make_float4(a.x + b.x, a.y + b.y, a.z + b.z, a.w + b.w); }
 // The same sixteen lanes that hold a column of a joint output tile reduce it (row = lane % 16 of the tile).
 __device__ __forceinline__ void tile_stat(float v, int tile, int row, int lane, bool ok, float4* stat, float* tail) {
     float m = row < kVocab ? v : -INFINITY;
@@ -376,6 +370,16 @@ __device__ __forceinline__ Share share_of(int phase, int n, int quad) {
     return {(int)(total * me / shares), (int)(total * (me + 1) / shares), groups};
 }
 
+// A cell's new state -> the candidate slot of sequence b.
+__device__ __forceinline__ void put_cell(const LoopState& L, size_t b, int slot, int layer, int unit, float cn, float hn) {
+    bf16 hi, lo;
+    split2(hn, hi, lo);
+    bf16* h = L.h + ((size_t)(slot * 2 + layer) * L.s.n_seq + b) * kRowElems + elem_of(unit);
+    __stcg(L.c + ((size_t)(slot * 2 + layer) * L.s.n_seq + b) * kH + unit, cn);
+    h[0] = hi;
+    h[8] = lo;
+}
+
 template <int PHASE>
 __device__ __forceinline__ void run_phase(const LoopState& L, Fragments& f, const uint32_t* list, int n, int quad, int qwarp, int lane,
                                           float (*sm)[kQuadWarps][16 * kPStride], size_t set = 0) {
@@ -414,26 +418,40 @@ __device__ __forceinline__ void run_phase(const LoopState& L, Fragments& f, cons
             f0 = __ldcg(list + min(next_n0 + g, n - 1));
             f1 = __ldcg(list + min(next_n0 + 8 + g, n - 1));
         }
-        // thread qt finishes row qt % 16 of columns qt / 16 (+ 8); what the epilogue adds is fetched under the product
+        // What the epilogue adds is fetched under the product.  Cells: threads of two of the four warps, by turns, finish unit
+        // qt % 4 of column (qt / 4) % 16, which is the column of one of their own list entries; other phases: thread qt
+        // finishes row qt % 16 of columns qt / 16 (+ 8).
+        const bool cells = PHASE == kPhaseB || (PHASE == kPhaseA && !rec);
+        const bool cell_warp = cells && (qwarp >> 1) == (item & 1);
+        const uint32_t ec = (qwarp & 1) ? e1 : e0;
+        const int unit = tile * 4 + (lane & 3);
+        float4 gates = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        float c_cell = 0.0f;
+        if (cell_warp) {
+            const size_t b = ec & kSeqMask;
+            if (PHASE == kPhaseA) {
+                gates = __ldg(reinterpret_cast<const float4*>(L.w.token_gates + (size_t)((ec >> kTokenShift) & kTokenMask) * kGates) + unit);
+                c_cell = __ldcg(L.c + (size_t)((ec >> 30) * 2) * BH + b * kH + unit);
+            } else {
+                gates = add4(__ldcg(reinterpret_cast<const float4*>(L.part + b * kGates) + unit), __ldg(reinterpret_cast<const float4*>(L.w.b1) + unit));
+                c_cell = __ldcg(L.c + (size_t)((ec >> 30) * 2 + 1) * BH + b * kH + unit);
+            }
+        }
         uint32_t e[2];
-        e[0] = __shfl_sync(0xffffffffu, e0, 4 * (qt >> 4));
-        e[1] = __shfl_sync(0xffffffffu, e1, 4 * (qt >> 4));
         float add[2], c_old[2];
+        if (!cells) {
+            e[0] = __shfl_sync(0xffffffffu, e0, 4 * (qt >> 4));
+            e[1] = __shfl_sync(0xffffffffu, e1, 4 * (qt >> 4));
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            const size_t b = e[j] & kSeqMask;
-            add[j] = c_old[j] = 0.0f;
-            if (PHASE == kPhaseA && !rec) {
-                add[j] = __ldg(L.w.token_gates + (size_t)((e[j] >> kTokenShift) & kTokenMask) * kGates + row);
-                c_old[j] = __ldcg(L.c + (size_t)((e[j] >> 30) * 2) * BH + b * kH + (row >> 2));
-            } else if (PHASE == kPhaseB) {
-                add[j] = __ldcg(L.part + b * kGates + row) + __ldg(L.w.b1 + row);
-                c_old[j] = __ldcg(L.c + (size_t)((e[j] >> 30) * 2 + 1) * BH + b * kH + (row >> 2));
-            } else if (PHASE == kPhaseC) {
-                add[j] = __ldg(L.b_pred + row);
-                c_old[j] = __ldg(s.enc_proj + (size_t)(s.enc_off[b] + __ldcg(s.frame_idx + b)) * kJointDim + row);
-            } else if (PHASE == kPhaseD) {
-                add[j] = __ldg(L.w.b_out + row);
+            for (int j = 0; j < 2; ++j) {
+                const size_t b = e[j] & kSeqMask;
+                add[j] = c_old[j] = 0.0f;
+                if (PHASE == kPhaseC) {
+                    add[j] = __ldg(L.b_pred + row);
+                    c_old[j] = __ldg(s.enc_proj + (size_t)(s.enc_off[b] + __ldcg(s.frame_idx + b)) * kJointDim + row);
+                } else if (PHASE == kPhaseD) {
+                    add[j] = __ldg(L.w.b_out + row);
+                }
             }
         }
         float v0[4], v1[4];
@@ -445,41 +463,37 @@ __device__ __forceinline__ void run_phase(const LoopState& L, Fragments& f, cons
         if (two) store_partial(P[qwarp], 1, lane, v1);
         if (more && next_tile != tile) fetch_fragments(f, tile_of(L.w, PHASE, next_tile), qwarp, lane);
         quad_barrier(quad);  // also: the other buffer's readers are done
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            if (j && !two) break;
-            const float val = sum_partials(P, ((qt >> 4) + 8 * j) * kPStride + r16) + add[j];
-            const size_t b = e[j] & kSeqMask;
-            const bool ok = n0 + (qt >> 4) + 8 * j < n;
-            if (PHASE == kPhaseA && rec) {
-                if (ok) __stcg(L.part + b * kGates + (row - kGates), val);
-            } else if (PHASE == kPhaseA || PHASE == kPhaseB) {
+        if (cells) {
+            const int col = (qt >> 2) & 15;
+            if (cell_warp && n0 + col < n) {
+                constexpr int layer = PHASE == kPhaseB ? 1 : 0;
                 float cn, hn;
-                cell(val, c_old[j], lane, cn, hn);
-                const int gate = lane & 3;
-                if (ok) {
-                    constexpr int layer = PHASE == kPhaseB ? 1 : 0;
-                    const int slot = (int)(e[j] >> 30) ^ 1, unit = row >> 2;
-                    bf16 hi, lo;
-                    split2(hn, hi, lo);
-                    bf16* ho = L.h + ((size_t)(slot * 2 + layer) * s.n_seq + b) * kRowElems + elem_of(unit);
-                    if (gate == 0) __stcg(L.c + (size_t)(slot * 2 + layer) * BH + b * kH + unit, cn);
-                    else if (gate == 1) ho[0] = hi;
-                    else if (gate == 2) ho[8] = lo;
-                }
-            } else if (PHASE == kPhaseC) {
-                if (ok) {
-                    bf16 hi, lo;
-                    split2(fmaxf(c_old[j] + val, 0.0f), hi, lo);
-                    __stcg(s.pred + b * kJointDim + row, val);
-                    L.z[b * kRowElems + elem_of(row)] = hi;
-                    L.z[b * kRowElems + elem_of(row) + 8] = lo;
-                }
-            } else {
-                tile_stat(val, tile, row, lane, ok, L.stat + (set * s.n_seq + b) * kOutTiles, L.tail + (set * s.n_seq + b) * 16);
-                if (ok && s.trace && row < kJointOut) {
-                    const int nsteps = __ldcg(s.n_steps + b);
-                    if (nsteps < s.trace_cap) s.trace[(b * s.trace_cap + nsteps) * kJointOut + row] = val;
+                cell(add4(sum_partials4(P, col * kPStride + 4 * (lane & 3)), gates), c_cell, cn, hn);
+                put_cell(L, ec & kSeqMask, (int)(ec >> 30) ^ 1, layer, unit, cn, hn);
+            }
+        } else {
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                if (j && !two) break;
+                const float val = sum_partials(P, ((qt >> 4) + 8 * j) * kPStride + r16) + add[j];
+                const size_t b = e[j] & kSeqMask;
+                const bool ok = n0 + (qt >> 4) + 8 * j < n;
+                if (PHASE == kPhaseA) {
+                    if (ok) __stcg(L.part + b * kGates + (row - kGates), val);
+                } else if (PHASE == kPhaseC) {
+                    if (ok) {
+                        bf16 hi, lo;
+                        split2(fmaxf(c_old[j] + val, 0.0f), hi, lo);
+                        __stcg(s.pred + b * kJointDim + row, val);
+                        L.z[b * kRowElems + elem_of(row)] = hi;
+                        L.z[b * kRowElems + elem_of(row) + 8] = lo;
+                    }
+                } else {
+                    tile_stat(val, tile, row, lane, ok, L.stat + (set * s.n_seq + b) * kOutTiles, L.tail + (set * s.n_seq + b) * 16);
+                    if (ok && s.trace && row < kJointOut) {
+                        const int nsteps = __ldcg(s.n_steps + b);
+                        if (nsteps < s.trace_cap) s.trace[(b * s.trace_cap + nsteps) * kJointOut + row] = val;
+                    }
                 }
             }
         }
@@ -633,10 +647,10 @@ tdt_decode_small_kernel(const __grid_constant__ LoopState L, int max_steps) {
     __shared__ Decision sh_dec[kSmallSeqs];
     __shared__ unsigned sh_live, sh_upd, sh_par;
     const DecodeState& s = L.s;
-    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, quad = warp / kQuadWarps, qwarp = warp % kQuadWarps;
-    const int n = s.n_seq;
+    const int tid = threadIdx.x, warp = tid >> 5, quad = warp / kQuadWarps, n = s.n_seq;
+    int lane = tid & 31, qwarp = warp % kQuadWarps;
     const bool two = n > 8;
-    const int me = quad * gridDim.x + blockIdx.x;
+    int me = quad * gridDim.x + blockIdx.x;
     const bool does_a = me < 2 * kLstmTiles, does_b = me < kLstmTiles;
     const bool does_d = !does_a && me < 2 * kLstmTiles + kOutTiles;
     const bool does_c = !does_a && !does_d && me < kSmallGroups;
@@ -665,86 +679,77 @@ tdt_decode_small_kernel(const __grid_constant__ LoopState L, int max_steps) {
         if (lane == 0) { sh_live = sh_upd = live; sh_par = 0; }
     }
     __syncthreads();
-    const int g = lane >> 2, q = lane & 3, qt = qwarp * 32 + lane, r16 = qt & 15;
-    const int colx[2] = {min(g, n - 1), min(8 + g, n - 1)};              // columns of this lane's operands
-    const int col[2] = {min(qt >> 4, n - 1), min(8 + (qt >> 4), n - 1)};  // columns this thread finishes
-    const bool mine[2] = {(qt >> 4) < n, 8 + (qt >> 4) < n};
-    float c0[2] = {0.0f, 0.0f}, c0_new[2] = {0.0f, 0.0f}, c1[2] = {0.0f, 0.0f}, c1_new[2] = {0.0f, 0.0f};
-
-    // product of this group's tile with the hidden vectors of `layer` (new: the candidates) -> P, summed by the caller
-    auto hidden_product = [&](int layer, bool fresh, unsigned par) {
-        float v[4];
-#pragma unroll
-        for (int j = 0; j < 2; ++j) {
-            if (j && !two) break;
-            const int slot = ((par >> colx[j]) & 1) ^ (fresh ? 1 : 0);
-            Pair x[kWarpKB];
-            load_x(x, L.h + ((size_t)(slot * 2 + layer) * n + colx[j]) * kRowElems + qwarp * kWarpKB * kBlockElems + q * 16);
-            product(f, x, v);
-            store_partial(P[quad][qwarp], j, lane, v);
-        }
-        quad_barrier(quad);
-    };
-    auto put_hidden = [&](int layer, int b, unsigned par, int unit, float hn) {
-        const int slot = ((par >> b) & 1) ^ 1;
-        bf16 hi, lo;
-        split2(hn, hi, lo);
-        bf16* ho = L.h + ((size_t)(slot * 2 + layer) * n + b) * kRowElems + elem_of(unit);
-        if ((lane & 3) == 1) ho[0] = hi;
-        else if ((lane & 3) == 2) ho[8] = lo;
-    };
+    float c0 = 0.0f, c0_new = 0.0f, c1 = 0.0f, c1_new = 0.0f;  // the state of this thread's cell
 
     for (int step = 0; step < max_steps; ++step) {
         const unsigned live = sh_live, upd = sh_upd, par = sh_par;
         if (live == 0) break;
         const size_t set = step & 1;
+        // what follows from these is formed anew in every step: kept for all of them, it takes more registers than there are
+        asm volatile("" : "+r"(lane), "+r"(qwarp), "+r"(me));
+        const int g = lane >> 2, q = lane & 3, qt = qwarp * 32 + lane, r16 = qt & 15;
+        const int colx[2] = {min(g, n - 1), min(8 + g, n - 1)};              // columns of this lane's operands
+        const int col[2] = {min(qt >> 4, n - 1), min(8 + (qt >> 4), n - 1)};  // columns this thread finishes
+        const bool mine[2] = {(qt >> 4) < n, 8 + (qt >> 4) < n};
+        const int ccol = min(qt >> 2, n - 1), cunit = qt & 3;  // the cell of threads 0 .. 4 n - 1 of a group: column, unit of the tile
+        const bool has_cell = qt < 4 * n;
+
+        // product of this group's tile with the hidden vectors of `layer` (new: the candidates) -> P, summed by the caller
+        auto hidden_product = [&](int layer, bool fresh, unsigned par) {
+            float v[4];
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+                if (j && !two) break;
+                const int slot = ((par >> colx[j]) & 1) ^ (fresh ? 1 : 0);
+                Pair x[kWarpKB];
+                load_x(x, L.h + ((size_t)(slot * 2 + layer) * n + colx[j]) * kRowElems + qwarp * kWarpKB * kBlockElems + q * 16);
+                product(f, x, v);
+                store_partial(P[quad][qwarp], j, lane, v);
+            }
+            quad_barrier(quad);
+        };
+        auto put_hidden = [&](int layer, unsigned par, int unit, float hn) {
+            const int slot = ((par >> ccol) & 1) ^ 1;
+            bf16 hi, lo;
+            split2(hn, hi, lo);
+            bf16* ho = L.h + ((size_t)(slot * 2 + layer) * n + ccol) * kRowElems + elem_of(unit);
+            ho[0] = hi;
+            ho[8] = lo;
+        };
         if (upd) {
             // ---- A
             if (does_a) {
                 const bool rec = me >= kLstmTiles;
-                const int row = me * 16 + r16;
-                float add[2] = {0.0f, 0.0f};
-                if (!rec) {
-                    add[0] = __ldg(L.w.token_gates + (size_t)sh_token[col[0]] * kGates + row);
-                    if (two) add[1] = __ldg(L.w.token_gates + (size_t)sh_token[col[1]] * kGates + row);
-                }
+                const int row = me * 16 + r16, unit = me * 4 + cunit;
+                float4 gates = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (!rec && has_cell) gates = __ldg(reinterpret_cast<const float4*>(L.w.token_gates + (size_t)sh_token[ccol] * kGates) + unit);
                 hidden_product(rec ? 1 : 0, false, par);
+                if (rec) {
 #pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    if (j && !two) break;
-                    const float v = sum_partials(P[quad], ((qt >> 4) + 8 * j) * kPStride + r16) + add[j];
-                    const bool ok = mine[j] && ((upd >> col[j]) & 1);
-                    if (rec) {
-                        if (ok) __stcg(L.part + (size_t)col[j] * kGates + (row - kGates), v);
-                    } else {
-                        float cn, hn;
-                        cell(v, c0[j], lane, cn, hn);
-                        if (ok) {
-                            c0_new[j] = cn;
-                            put_hidden(0, col[j], par, row >> 2, hn);
-                        }
+                    for (int j = 0; j < 2; ++j) {
+                        if (j && !two) break;
+                        const float v = sum_partials(P[quad], ((qt >> 4) + 8 * j) * kPStride + r16);
+                        if (mine[j] && ((upd >> col[j]) & 1)) __stcg(L.part + (size_t)col[j] * kGates + (row - kGates), v);
                     }
+                } else if (has_cell && ((upd >> ccol) & 1)) {
+                    float hn;
+                    cell(add4(sum_partials4(P[quad], ccol * kPStride + 4 * cunit), gates), c0, c0_new, hn);
+                    put_hidden(0, par, unit, hn);
                 }
                 if (does_b) fetch_fragments(f, tile_b, qwarp, lane);
             }
             if (!grid.sync()) return;
             // ---- B
             if (does_b) {
-                const int row = me * 16 + r16;
-                float add[2];
-                add[0] = __ldcg(L.part + (size_t)col[0] * kGates + row) + __ldg(L.w.b1 + row);
-                add[1] = two ? __ldcg(L.part + (size_t)col[1] * kGates + row) + __ldg(L.w.b1 + row) : 0.0f;
+                const int unit = me * 4 + cunit;
+                float4 gates = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if (has_cell)
+                    gates = add4(__ldcg(reinterpret_cast<const float4*>(L.part + (size_t)ccol * kGates) + unit), __ldg(reinterpret_cast<const float4*>(L.w.b1) + unit));
                 hidden_product(0, true, par);
-#pragma unroll
-                for (int j = 0; j < 2; ++j) {
-                    if (j && !two) break;
-                    const float v = sum_partials(P[quad], ((qt >> 4) + 8 * j) * kPStride + r16) + add[j];
-                    float cn, hn;
-                    cell(v, c1[j], lane, cn, hn);
-                    if (mine[j] && ((upd >> col[j]) & 1)) {
-                        c1_new[j] = cn;
-                        put_hidden(1, col[j], par, row >> 2, hn);
-                    }
+                if (has_cell && ((upd >> ccol) & 1)) {
+                    float hn;
+                    cell(add4(sum_partials4(P[quad], ccol * kPStride + 4 * cunit), gates), c1, c1_new, hn);
+                    put_hidden(1, par, unit, hn);
                 }
                 fetch_fragments(f, tile_a, qwarp, lane);
             }
@@ -839,12 +844,10 @@ tdt_decode_small_kernel(const __grid_constant__ LoopState L, int max_steps) {
         }
         __syncthreads();
         const unsigned emitted = par ^ sh_par;
-#pragma unroll
-        for (int j = 0; j < 2; ++j)
-            if ((emitted >> col[j]) & 1) {
-                c0[j] = c0_new[j];
-                c1[j] = c1_new[j];
-            }
+        if ((emitted >> ccol) & 1) {
+            c0 = c0_new;
+            c1 = c1_new;
+        }
     }
     if (blockIdx.x == 0 && tid < n) {
         s.n_tokens[tid] = sh_tokens[tid];

@@ -144,3 +144,33 @@ def test_batch_sizes_around_the_kernel_lines(ctx, weights, n):
             assert np.array_equal(g[k], h[k])
             if k != "conf":
                 assert np.array_equal(rep[k], g[k])
+
+
+def test_small_cell_states_keep_their_digits(ctx, weights):
+    """Candidate gates near zero (rows of the third gate scaled by 1e-4, the predictor's projection by 1e6): the hyperbolic
+    tangent must be exact relative to its own size there.  Formed as a difference from one it has an absolute error of 2^-24
+    or more, 1e-2 of these states and of the logits; the first step's logits are held to 2e-4 of 64-bit arithmetic: the split
+    products drop 2^-16 of |x||w| in each of the chain's four, the functions and sums some 2^-21."""
+    import scriptrs_b200 as sb
+
+    w = {k: v.copy() for k, v in weights.items()}
+    third = slice(2 * 640, 3 * 640)
+    for k in ("weight_ih", "weight_hh", "bias_ih", "bias_hh"):
+        w["predictor.lstm." + k][:, third] *= np.float32(1e-4)
+    w["joint.pred.weight"] *= np.float32(1e6)
+    enc = np.random.default_rng(11).standard_normal((1, 1024)).astype(np.float32)
+    try:
+        sb.load_model(ctx, w, encoder_layers=0, has_encoder=False, has_decoder=True)
+        got = [decode_gpu(ctx, [enc] * n)[-1]["logits"][0] for n in (1, 17)]  # both kernels' cells
+    finally:
+        sb.load_model(ctx, weights, encoder_layers=0, has_encoder=False, has_decoder=True)
+    d = {k: v.astype(np.float64) for k, v in w.items()}
+    x = d["predictor.embedding"][1024]
+    for layer in range(2):
+        g = d["predictor.lstm.weight_ih"][layer] @ x + d["predictor.lstm.bias_ih"][layer] + d["predictor.lstm.bias_hh"][layer]
+        i, _, c, o = np.split(g, 4)
+        x = np.tanh(np.tanh(c) / (1.0 + np.exp(-i))) / (1.0 + np.exp(-o))
+    z = d["joint.enc.weight"] @ enc[0] + d["joint.enc.bias"] + d["joint.pred.weight"] @ x + d["joint.pred.bias"]
+    ref = d["joint.out.weight"] @ np.maximum(z, 0.0) + d["joint.out.bias"]
+    for logits in got:
+        assert np.linalg.norm(logits - ref) / np.linalg.norm(ref) < 2e-4
