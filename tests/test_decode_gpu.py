@@ -174,3 +174,70 @@ def test_small_cell_states_keep_their_digits(ctx, weights):
     ref = d["joint.out.weight"] @ np.maximum(z, 0.0) + d["joint.out.bias"]
     for logits in got:
         assert np.linalg.norm(logits - ref) / np.linalg.norm(ref) < 2e-4
+
+
+@pytest.mark.parametrize("blank_bias", [0.0, 1.5])
+@pytest.mark.parametrize("n", [383, 384, 401, 1000])
+def test_large_batches_equal_small_ones(ctx, weights, decode_path, n, blank_bias):
+    """The largest batch of the kernel for some hundred sequences, and the one for more (its smallest, a last group of one column,
+    more than one block of tiles per thread block): clips of 0 to 12 frames, with an emission in nearly every step or with blanks
+    in most.  Tokens, confidences and logits equal those of the same clips in batches of 100, bit for bit, and their replay."""
+    import scriptrs_b200 as sb
+
+    if decode_path == "simt":
+        pytest.skip("the lines are those of the tensor-core decoder")
+    w = dict(weights)
+    w["joint.out.bias"] = weights["joint.out.bias"].copy()
+    w["joint.out.bias"][1024] += np.float32(blank_bias)
+    rng = np.random.default_rng(n)
+    encs = [rng.standard_normal((int(t), 1024)).astype(np.float32) for t in rng.integers(0, 13, size=n)]
+    try:
+        sb.load_model(ctx, w, encoder_layers=0, has_encoder=False, has_decoder=True)
+        got = decode_gpu(ctx, encs)
+        small = [g for i in range(0, n, 100) for g in decode_gpu(ctx, encs[i:i + 100])]
+    finally:
+        sb.load_model(ctx, weights, encoder_layers=0, has_encoder=False, has_decoder=True)
+    for i, (g, h) in enumerate(zip(got, small)):
+        assert g["steps"] == h["steps"]
+        for k in ("tokens", "frames", "durations", "conf"):
+            assert np.array_equal(g[k], h[k]), (i, k)
+        assert np.array_equal(g["logits"], h["logits"]), i
+        if i % 17 == 0 and encs[i].shape[0]:
+            rep = oracle.greedy_replay(g["logits"], time_steps=encs[i].shape[0])
+            assert rep["steps"] == g["steps"] and all(np.array_equal(rep[k], g[k]) for k in ("tokens", "frames", "durations"))
+
+
+def test_two_contexts_decode_at_the_same_time(ctx, weights, decode_path):
+    """The decoder's grid occupies every SM and waits for itself.  Two host threads with a context each keep it busy with batches
+    of all three kernels: every call must return what it returns alone."""
+    import threading
+
+    import scriptrs_b200 as sb
+
+    rng = np.random.default_rng(5)
+    batches = [[rng.standard_normal((int(t), 1024)).astype(np.float32) for t in rng.integers(1, 30, size=n)] for n in (400, 5, 60)]
+    second = sb.Context(0)
+    try:
+        second.set_option("simt_decode", 1 if decode_path == "simt" else 0)
+        sb.load_model(second, weights, encoder_layers=0, has_encoder=False, has_decoder=True)
+        alone = [decode_gpu(ctx, b, trace=False) for b in batches]
+        results, errors = {}, []
+
+        def work(who, c):
+            try:
+                for i in range(12):
+                    results[who, i] = decode_gpu(c, batches[(i + who) % 3], trace=False)
+            except Exception as e:  # noqa: BLE001
+                errors.append(e)
+
+        threads = [threading.Thread(target=work, args=(k, c)) for k, c in enumerate((ctx, second))]
+        for t in threads:
+            t.start()
+        for t in threads:
+            t.join()
+        assert not errors, errors
+        for (who, i), got in results.items():
+            for g, a in zip(got, alone[(i + who) % 3]):
+                assert all(np.array_equal(g[k], a[k]) for k in ("tokens", "frames", "durations", "conf"))
+    finally:
+        second.close()
