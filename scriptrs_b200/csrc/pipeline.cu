@@ -32,7 +32,8 @@ void decode_workspace_free(sb_ctx* c) {
     }
 }
 
-constexpr int kMaxSeqPerLaunch = 8192;  // the kernel keeps two index lists of this many ints in shared memory
+// Thirteen bits of the tensor-core decoder's list entries; the fp32 kernel keeps two lists of this many ints in shared memory.
+constexpr int kMaxSeqPerLaunch = 8192;
 
 int32_t tdt_decode(sb_ctx* c, const float* d_enc, const int64_t* enc_offsets, int64_t n_clips, int64_t max_tokens,
                    uint32_t* token_ids, int64_t* frame_indices, int64_t* durations, float* confidences,
@@ -70,12 +71,13 @@ int32_t tdt_decode(sb_ctx* c, const float* d_enc, const int64_t* enc_offsets, in
         std::memcpy(hi.data() + n, len.data(), sizeof(int) * n);
         for (int i = 0; i < n; ++i) hi[(size_t)4 * n + i] = kVocab - 1;  // last_token = blank (model.rs:123)
         SB_CUDA(cudaMemcpyAsync(di, hi.data(), n_int * sizeof(int), cudaMemcpyHostToDevice, st));
-        // float state: h, c, h_new, c_new [2][n][640], pred [n][640], logits [n][1030]
-        const size_t BH = (size_t)n * kPredHidden;
-        const size_t n_f = 8 * BH + 2 * (size_t)n * kJointDim + (size_t)n * kJointOut;
-        SB_CUDA(ws.floats.ensure(n_f * sizeof(float)));
+        // float state: pred [n][640]; the fp32 kernel also keeps h, c, h_new, c_new [2][n][640], z [n][640] and logits [n][1030]
+        // here, the tensor-core decoder its own in the scratch area
+        const bool tc = !c->simt_decode;
+        const size_t BH = (size_t)n * kPredHidden, n_pred = (size_t)n * kJointDim;
+        SB_CUDA(ws.floats.ensure((tc ? n_pred : 8 * BH + 2 * n_pred + (size_t)n * kJointOut) * sizeof(float)));
         float* df = ws.floats.as<float>();
-        if (c->simt_decode) SB_CUDA(cudaMemsetAsync(df, 0, 4 * BH * sizeof(float), st));  // h = c = 0 (model.rs:114-115)
+        if (!tc) SB_CUDA(cudaMemsetAsync(df + n_pred, 0, 4 * BH * sizeof(float), st));  // h = c = 0 (model.rs:114-115)
         SB_CUDA(ws.enc_proj.ensure((size_t)std::max<int64_t>(rows, 1) * kJointDim * sizeof(float)));
         SB_CUDA(ws.out_tok.ensure((size_t)n * max_tokens * sizeof(uint32_t)));
         SB_CUDA(ws.out_frm.ensure((size_t)n * max_tokens * sizeof(int)));
@@ -83,7 +85,6 @@ int32_t tdt_decode(sb_ctx* c, const float* d_enc, const int64_t* enc_offsets, in
         SB_CUDA(ws.out_conf.ensure((size_t)n * max_tokens * sizeof(float)));
         if (logits_trace) SB_CUDA(ws.trace.ensure((size_t)n * trace_cap * kJointOut * sizeof(float)));
 
-        const bool tc = !c->simt_decode;
         if (tc) {
             SB_CUDA(ws.tc.ensure(decode_tc_scratch_bytes(rows, n)));
             c->prof.begin("decode_enc_projection_tc", st);
@@ -112,22 +113,24 @@ int32_t tdt_decode(sb_ctx* c, const float* d_enc, const int64_t* enc_offsets, in
         s.n_tokens = di + 6 * n;
         s.n_steps = di + 7 * n;
         s.overflow = di + 8 * n;
-        s.h = df;
-        s.c = df + 2 * BH;
-        s.h_new = df + 4 * BH;
-        s.c_new = df + 6 * BH;
-        s.pred = df + 8 * BH;
-        s.z = s.pred + (size_t)n * kJointDim;
-        s.logits = s.z + (size_t)n * kJointDim;
+        s.pred = df;
+        if (!tc) {
+            s.h = df + n_pred;
+            s.c = s.h + 2 * BH;
+            s.h_new = s.h + 4 * BH;
+            s.c_new = s.h + 6 * BH;
+            s.z = s.h + 8 * BH;
+            s.logits = s.z + n_pred;
+        }
         s.out_tokens = ws.out_tok.as<uint32_t>();
         s.out_frames = ws.out_frm.as<int>();
         s.out_durs = ws.out_dur.as<int>();
         s.out_conf = ws.out_conf.as<float>();
         s.trace = logits_trace ? ws.trace.as<float>() : nullptr;
-        // SB_DECODE_TIMING=1: block 0's cycle counts per phase / barrier, printed after the kernel
+        // SB_DECODE_TIMING=1: block 0's cycle counts per phase / barrier, printed after the fp32 kernel
         static const bool want_timing = std::getenv("SB_DECODE_TIMING") != nullptr;
         long long* d_timing = nullptr;
-        if (want_timing) {
+        if (want_timing && !tc) {
             SB_CUDA(ws.timing.ensure(12 * sizeof(long long)));
             d_timing = ws.timing.as<long long>();
             SB_CUDA(cudaMemsetAsync(d_timing, 0, 12 * sizeof(long long), st));
