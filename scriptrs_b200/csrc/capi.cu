@@ -135,7 +135,7 @@ int32_t frontend_run(sb_ctx* c, const void* d_pcm, SampleFormat fmt, const int64
     const int64_t* d_meta = c->clip_off.as<int64_t>();
     c->prof.begin("frontend", c->stream);
     cudaError_t e = frontend_launch(d_pcm, fmt, d_meta, d_meta + n1, d_meta + 2 * n1, (int)n_clips, fo[n_clips], max_frames, preemphasis,
-                                    c->d_tables, d_feats, normalize, c->stream, &c->launches);
+                                    c->d_tables, d_feats, normalize, c->sm_count, c->stream, &c->launches);
     c->prof.end(c->stream);
     if (e == cudaErrorMisalignedAddress)
         return fail(SB_INVALID_ARGUMENT, "the feature buffer must be 16-byte aligned and the PCM buffer aligned to its sample type");

@@ -443,33 +443,41 @@ cudaError_t norm_launch(const int64_t* d_frame_off, int n_clips, int max_frames,
 template <typename TIn>
 cudaError_t launch_format(const TIn* pcm, const int64_t* d_clip_start, const int64_t* d_clip_len, const int64_t* d_frame_off,
                           int n_clips, int64_t total_frames, int max_frames, float preemph, const FrontendTables* d_tables,
-                          float* feats, bool normalize, cudaStream_t stream, int64_t* launches) {
+                          float* feats, bool normalize, int sm_count, cudaStream_t stream, int64_t* launches) {
     *launches += 1;
-    // One CTA per clip, or the clip's steps and columns spread over the chip.  Measured on clips of 1501 frames
-    // (one-CTA kernel / split, us): 1 clip 304 / 31, 16 clips 304 / 54, 97 ragged clips 307 / 165, 148 clips
-    // 335 / 296, 200 clips 453 / 424, 296 clips 489 / 576; on 3001 frames: 1 clip 598 / 44, 148 clips 663 / 676.  The
-    // one-CTA kernel takes 0.2 us per frame of the longest clip until the SMs are full, the split 1.4 ns per frame in
-    // all, so the line lies where the batch holds about 128 clips' worth of the longest one.  A clip of one or two
-    // steps has nothing to split, and the column blocks of a longer one than kSplitMaxFrames do not fit.
+    // One CTA per clip, or the clip's steps and columns spread over the chip.  The one-CTA kernel takes 0.205 us per frame of
+    // the longest clip until the SMs are full; the split 1.35 ns per frame in all on 148 SMs, 5 us for its second
+    // launch, and 4.5 us for every further wave of that launch's CTAs, whose shared memory is sized for the longest clip: a long
+    // clip among thousands of short ones makes them many.  Measured (one-CTA kernel / split, us): 1 clip of 1501 frames
+    // 304 / 31, 97 ragged ones 307 / 153, 127 330 / 276, 96 clips of 64 frames 21.5 / 23.9, of 101 frames 31 / 30, of 401 93 /
+    // 62; one clip of 3594 frames with 2000 of 51 757 / 609, with 4000 of 101 838 / 1650, with 40000 of 11 frames 960 / 7100.
+    // From 148 clips of one length the two lie within 12 % of one another, on either side (1501 frames: 148 clips 335 /
+    // 296, 200 clips 453 / 424, 296 clips 489 / 576; 3001 frames: 148 clips 663 / 676): the rule leaves them on one launch.
+    // A clip of one or two steps has nothing to split, and the column blocks of a longer one than kSplitMaxFrames do
+    // not fit.
+    const int cols = max_frames <= kSplitMaxFrames / 2 ? 32 : 16;
+    const int64_t norm_smem = (int64_t)max_frames * cols * (int)sizeof(float);
+    const int64_t slots = sm_count * std::max<int64_t>(1, std::min<int64_t>(8, 227 * 1024 / (norm_smem + 1024)));
+    const int64_t waves = normalize ? ((int64_t)(kMels / cols) * n_clips + slots - 1) / slots : 1;
     const bool split = max_frames > 2 * kStepFrames && max_frames <= kSplitMaxFrames && n_clips <= 65535 &&
-                       total_frames < (int64_t)128 * max_frames;
+                       5.0 + 1.35e-3 * 148.0 / sm_count * total_frames + 4.5 * (waves - 1) < 0.205 * max_frames;
     if (!split) {
         frontend_clip_kernel<TIn, false><<<n_clips, kThreads, sizeof(SmemLayout), stream>>>(
             pcm, d_clip_start, d_clip_len, d_frame_off, feats, preemph, d_tables, normalize ? 1 : 0, 0);
         return cudaGetLastError();
     }
     const int max_steps = (max_frames + kStepFrames - 1) / kStepFrames;
-    // steps per CTA: four CTAs per resident slot if the batch gives as many (the tables are loaded once per CTA; one
-    // step per CTA is 15 % slower on 97 clips), and a bounded number of CTAs that find their clip already over
+    // steps per CTA: four CTAs for each of an SM's two places if the batch gives as many (the tables are loaded once per
+    // CTA; one step per CTA is 15 % slower on 97 clips), and a bounded number of CTAs that find their clip already over
     const int64_t steps = total_frames / kStepFrames + n_clips;
-    const int chunk = (int)std::max(std::min<int64_t>(16, std::max<int64_t>(1, steps / 1184)), (max_steps * (int64_t)n_clips + 16383) / 16384);
+    const int chunk = (int)std::max(std::min<int64_t>(16, std::max<int64_t>(1, steps / (8 * sm_count))), (max_steps * (int64_t)n_clips + 16383) / 16384);
     frontend_clip_kernel<TIn, true><<<dim3((max_steps + chunk - 1) / chunk, n_clips), kThreads, sizeof(SmemLayout), stream>>>(
         pcm, d_clip_start, d_clip_len, d_frame_off, feats, preemph, d_tables, 0, chunk);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess || !normalize) return e;
     *launches += 1;
-    return max_frames <= kSplitMaxFrames / 2 ? norm_launch<32>(d_frame_off, n_clips, max_frames, feats, stream)
-                                                                   : norm_launch<16>(d_frame_off, n_clips, max_frames, feats, stream);
+    return cols == 32 ? norm_launch<32>(d_frame_off, n_clips, max_frames, feats, stream)
+                      : norm_launch<16>(d_frame_off, n_clips, max_frames, feats, stream);
 }
 
 }  // namespace
@@ -491,7 +499,7 @@ cudaError_t frontend_configure() {
 
 cudaError_t frontend_launch(const void* pcm, SampleFormat fmt, const int64_t* d_clip_start, const int64_t* d_clip_len,
                             const int64_t* d_frame_off, int n_clips, int64_t total_frames, int max_frames, float preemph,
-                            const FrontendTables* d_tables, float* feats, bool normalize, cudaStream_t stream,
+                            const FrontendTables* d_tables, float* feats, bool normalize, int sm_count, cudaStream_t stream,
                             int64_t* launches) {
     int64_t ignored;
     if (!launches) launches = &ignored;
@@ -501,9 +509,9 @@ cudaError_t frontend_launch(const void* pcm, SampleFormat fmt, const int64_t* d_
         return cudaErrorMisalignedAddress;
     if (fmt == kSampleI16)
         return launch_format(static_cast<const int16_t*>(pcm), d_clip_start, d_clip_len, d_frame_off, n_clips, total_frames,
-                             max_frames, preemph, d_tables, feats, normalize, stream, launches);
+                             max_frames, preemph, d_tables, feats, normalize, sm_count, stream, launches);
     return launch_format(static_cast<const float*>(pcm), d_clip_start, d_clip_len, d_frame_off, n_clips, total_frames,
-                         max_frames, preemph, d_tables, feats, normalize, stream, launches);
+                         max_frames, preemph, d_tables, feats, normalize, sm_count, stream, launches);
 }
 
 }  // namespace sb

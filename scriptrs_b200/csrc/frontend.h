@@ -55,7 +55,7 @@ cudaError_t frontend_configure();
 // two that spread each clip over several CTAs; *launches is advanced by their number.
 cudaError_t frontend_launch(const void* pcm, SampleFormat fmt, const int64_t* d_clip_start, const int64_t* d_clip_len,
                             const int64_t* d_frame_off, int n_clips, int64_t total_frames, int max_frames, float preemph,
-                            const FrontendTables* d_tables, float* feats, bool normalize, cudaStream_t stream,
+                            const FrontendTables* d_tables, float* feats, bool normalize, int sm_count, cudaStream_t stream,
                             int64_t* launches = nullptr);
 
 }  // namespace sb

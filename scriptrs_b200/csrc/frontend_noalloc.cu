@@ -134,8 +134,11 @@ extern "C" int32_t sb_frontend_device_noalloc(const float* d_pcm, const int64_t*
     // pageable source: the runtime has staged the bytes by the time the call returns
     e = cudaMemcpyAsync(d_meta, meta, sizeof(meta), cudaMemcpyHostToDevice, st);
     if (e != cudaSuccess) return cuda_fail(e, "copy of the clip metadata");
+    int sm_count = 0;
+    e = cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, device);
+    if (e != cudaSuccess) return cuda_fail(e, "cudaDeviceGetAttribute");
     e = frontend_launch(d_pcm, kSampleF32, d_meta, d_meta + n1, d_meta + 2 * n1, (int)n_clips, fo[n_clips], max_frames, preemphasis, d_tables,
-                        d_feats, normalize != 0, st);
+                        d_feats, normalize != 0, sm_count, st);
     if (e == cudaErrorMisalignedAddress) return fail(SB_INVALID_ARGUMENT, "the feature buffer must be 16-byte aligned");
     if (e != cudaSuccess) return cuda_fail(e, "frontend launch");
     return SB_OK;
