@@ -152,15 +152,16 @@ int64_t sb_ctx_kernel_launches(const sb_ctx* ctx);
  * "simt_subsample" (0/1): run the first two sub-sampling stages in fp32 on CUDA cores instead of the fp16
  * tensor-core kernel.  "simt_attention" (0/1): run the relative-position attention on CUDA cores
  * instead of the tensor-core kernel; "simt_decode" (0/1): run the TDT predictor and joint in plain fp32 on
- * CUDA cores (one persistent kernel) instead of the split-bf16 tensor-core steps; "gemm_pair_tiles" (0/1/2,
+ * CUDA cores (one persistent kernel) instead of the split-bf16 tensor-core products; "gemm_pair_tiles" (0/1/2,
  * process-wide): two-CTA 256 x 256 GEMM tiles never / where they pay (default) / wherever they fit;
  * "vad_unstreamed" (0/1): in the VAD long-form mode run the whole voice-activity network before the first
  * transcription kernel instead of beside the transcription; "vad_rows_cap" (default 0 = sized from the recording): encoder
  * frames the streamed VAD mode keeps before it runs the decoder over them (more tasks than fit are decoded in rounds);
  * "vad_stream_pass_windows" (default 49152): largest pass of the network in the streamed VAD mode;
  * "vad_cluster" (4 or 8, default 8): thread blocks in the cluster that runs the VAD network's recurrence;
- * "vad_segment_windows" (default 131072): windows the VAD network processes per pass (its work buffers hold 2560 bytes
- * per window; the recurrent state is carried from pass to pass);
+ * "vad_segment_windows" (default 131072): windows the VAD network's work buffers hold (at most 2560 bytes per window; the
+ * recurrent state is carried from pass to pass): one pass of that many on a device-resident recording, two of half as many,
+ * by turns, where passes are copied in under the recurrence (sb_vad_process);
  * "workspace_budget_mb":
  * MB of encoder intermediates per group of clips (default 49152: the 2236 chunks of an 8 h recording form one group; a
  * batch allocates only what it needs). */

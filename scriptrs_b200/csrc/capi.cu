@@ -495,7 +495,8 @@ int32_t sb_vad_process(sb_ctx* c, const float* audio, int64_t n_samples, float* 
     // From pageable memory a window's 2 KB cross PCIe in half the 0.35 us that its step of the recurrence takes, so each
     // pass of a doubling sequence is copied while the one before it recurs, and only the first, short one is exposed.
     VadPasses passes;
-    int32_t s = passes.begin(c, audio, n_samples, 1024, std::min(c->vad_segment_windows, 32768));
+    // Two passes' gate inputs are held at once: each takes half of the windows that "vad_segment_windows" allows.
+    int32_t s = passes.begin(c, audio, n_samples, 1024, std::max(1, c->vad_segment_windows / 2));
     for (int k = 0; s == SB_OK && k < passes.count(); ++k) s = passes.enqueue(k);
     if (s != SB_OK) {
         const std::string why = sb_last_error();

@@ -268,3 +268,32 @@ def test_vad_mode_with_two_contexts(ctx, pipe):
         assert second.kernel_launches() > k0 and len(one.token_ids) > 0
     finally:
         second.close()
+
+
+def test_segment_option_bounds_the_passes_of_a_host_recording(ctx):
+    """"vad_segment_windows" sets the size of the passes over its whole range (values above 32768 windows included): 1024 windows,
+    then doubling up to half of it.  The probabilities do not depend on it."""
+    import scriptrs_b200 as sb
+
+    net = sb.SileroVad(ctx, synth.seeded_vad_weights(5))
+    audio = np.random.default_rng(3).standard_normal(100_000 * 512).astype(np.float32) * np.float32(0.05)
+
+    def passes(largest):
+        sizes, left = [], 100_000
+        while left > 0:
+            sizes.append(min(left, largest, 1024 << len(sizes)))
+            left -= sizes[-1]
+        return len(sizes)
+
+    got = {}
+    try:
+        for option in (131072, 65536, 9000):
+            ctx.set_option("vad_segment_windows", option)
+            before = ctx.kernel_launches()
+            got[option] = net.process(audio)
+            assert ctx.kernel_launches() - before == 3 * passes(option // 2), option
+    finally:
+        ctx.set_option("vad_segment_windows", 131072)
+    assert passes(65536) < passes(32768) < passes(4500)
+    for p in got.values():
+        assert p.size == 100_000 and np.array_equal(p, got[131072])
