@@ -657,7 +657,7 @@ static cudaError_t encode_group(sb_ctx* c, const Model& m, const float* d_feats,
                                                                                        m.dw1_w, m.dw1_b, ws.y1.as<bf16>())));
         } else {
             c->prof.begin("sub_conv0_dw1", st);
-            ENC_CUDA(subsample_conv0_dw1_launch(d_feats, d_t0, d_t1, d_t2, n, max_t2, m.sub0_frag, m.dw1_pairs, ws.y1.p, st));
+            ENC_CUDA(subsample_conv0_dw1_launch(d_feats, d_t0, d_t1, d_t2, n, max_t2, m.sub0_frag, m.dw1_pairs, ws.y1.p, c->sm_count, st));
             c->prof.end(st);
         }
         c->launches += 1;

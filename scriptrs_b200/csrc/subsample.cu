@@ -15,8 +15,8 @@
 //             padding), 16-byte stores into a [5 rows x 65 columns x 64 channels] tile (column slot 0 = padding)
 //   depthwise each thread owns four channels and two output frequencies and slides a 5 x 5 window over
 //             the tile; fp16 multiply-adds (the result is rounded to bf16 anyway), 8-byte bf16 stores
-// Bound by shared-memory wavefronts (the first-stage tile is written and read once per row and block: 3900 a step, L1 at
-// 90 % of its peak; 560 clips of 1497 frames 3.03 -> 2.70 ms against 4-byte stores, two channels a thread and no prefetch,
+// Bound by shared-memory wavefronts (the first-stage tile is written and read once per row and block: 3900 a step; 560 clips
+// of 1497 frames 3.03 -> 2.70 ms against 4-byte stores, two channels a thread and no prefetch,
 // which took 15.6 k warp instructions a step instead of 11.8 k).
 // fp16 keeps 11 significant bits of the normalised features and of the weights; the accumulation of the first stage
 // is fp32.
@@ -259,11 +259,11 @@ cudaError_t subsample_configure() {
 }
 
 cudaError_t subsample_conv0_dw1_launch(const float* feats, const int64_t* d_t0, const int* d_t1, const int* d_t2, int n_clips,
-                                       int max_t2, const void* w0_frag, const void* w1_pairs, void* out, cudaStream_t st) {
+                                       int max_t2, const void* w0_frag, const void* w1_pairs, void* out, int sm_count, cudaStream_t st) {
     if (n_clips <= 0 || max_t2 <= 0) return cudaSuccess;
     // four steps of two rows per CTA while that leaves four CTAs for each of the three places on an SM
     const int pairs = (max_t2 + kTO - 1) / kTO;
-    const int steps = (int64_t)pairs * n_clips >= (int64_t)4 * 12 * 148 ? 4 : 1;
+    const int steps = (int64_t)pairs * n_clips >= (int64_t)4 * 12 * sm_count ? 4 : 1;
     const dim3 grid((pairs + steps - 1) / steps, n_clips);
     if (reinterpret_cast<uintptr_t>(feats) & 3) return cudaErrorMisalignedAddress;
     auto* kernel = reinterpret_cast<uintptr_t>(feats) & 15 ? sub_conv0_dw1_tc_kernel<4> : sub_conv0_dw1_tc_kernel<16>;
