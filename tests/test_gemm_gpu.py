@@ -144,3 +144,31 @@ def test_a_row_does_not_depend_on_the_tile_width(ctx, N, K, act, out_mode):
     acc = a[:376].float() @ w.float().t() + bias
     ref = ref_epilogue(acc, None, act) + (3.0 if out_mode == 2 else 0.0)
     assert (whole[:376].float() - ref).norm() / ref.norm() < (6e-3 if dtype == torch.bfloat16 else 1e-4)
+
+
+def test_glu_rows_do_not_depend_on_the_tile_width(ctx):
+    """The gated epilogue leaves 64-byte slabs from 64- and 128-column tiles and 128-byte ones from wider tiles: rows of a product of
+    any size are equal bit for bit, nothing beyond the last row or the N / 2 output columns is written, and the values are those
+    of a float32 reference."""
+    import scriptrs_b200 as sb
+
+    N, K, most = 2048, 1024, 4500
+    g = torch.Generator(device="cuda").manual_seed(3)
+    a = (torch.randn(most, K, device="cuda", generator=g) * 0.5).to(torch.bfloat16)
+    w = (torch.randn(N, K, device="cuda", generator=g) * 0.05).to(torch.bfloat16)
+    bias = torch.randn(N, device="cuda", generator=g) * 0.1
+
+    def run(m):
+        out = torch.full((m + 1, N), 3.0, device="cuda", dtype=torch.bfloat16)
+        torch.cuda.synchronize()
+        sb.gemm(ctx, a.data_ptr(), w.data_ptr(), out.data_ptr(), m, N, K, d_bias=bias.data_ptr(), act=3, out_mode=0)
+        ctx.synchronize()
+        assert (out[m] == 3.0).all() and (out[:, N // 2:] == 3.0).all()
+        return out[:m, :N // 2]
+
+    whole = run(most)
+    for m in (1, 127, 188, 512, 513, 640, 1000, 1152, 1153, 2304):
+        assert torch.equal(run(m), whole[:m]), m
+    v, gate = (a.float() @ w.float().t() + bias).reshape(most, N // 32, 2, 16).unbind(2)
+    ref = (v * torch.sigmoid(gate)).reshape(most, N // 2)
+    assert (whole.float() - ref).norm() / ref.norm() < 4e-3  # one rounding to bf16: 2^-9 each, 2^-9 / sqrt(3) in the norm
