@@ -9,7 +9,7 @@
 //   warp 0      TMA producer: 128-byte-swizzled [128 x 64] A tiles and [BN x 64] W tiles
 //               through a multi-stage shared-memory ring (full / empty mbarriers)
 //   warp 1      allocates tensor memory, issues tcgen05.mma (M = 128, N = BN, K = 16 per
-//               instruction, four per stage) from one lane; tcgen05.commit releases ring
+//               instruction, four per stage) from one elected lane; tcgen05.commit releases ring
 //               slots and publishes finished accumulators
 //   warps 2..9  epilogue: each warp owns one 32-lane quadrant of tensor memory and one half of
 //               the tile's columns; tcgen05.ld (one row per thread), scales / bias / activation,
