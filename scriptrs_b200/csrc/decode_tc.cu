@@ -647,8 +647,8 @@ tdt_decode_tc_kernel(const __grid_constant__ LoopState L, int max_steps) {
 // its MMAs about two cycles; a second group for the epilogues changes nothing.  The loop alone against the kernel above, ms
 // with blanks in most steps / with an emission in nearly every step: 280 sequences 5.2 / 16.3 against 5.0 / 16.1, 400 5.7 / 19.4
 // against 5.9 / 20.1, 1120 10.3 / 39 against 11.5 / 44, 2236 18.2 / 72 against 20.4 / 81: the line lies between the first two.
-// (Weights of 64 rows in shared memory and activations in registers: 92 at 2236; this layout without the third group 107; four
-// groups of one tile 125.)  The sums are those of the other kernels, term by term: a sequence's numbers do not depend on the
+// (At 2236, all with an emission in nearly every step: weights of 64 rows in shared memory and activations in registers 76; this
+// layout with the copies and epilogues in the product groups 101; four such groups of one tile each 105.)  The sums are those of the other kernels, term by term: a sequence's numbers do not depend on the
 // kernel that its batch took.
 constexpr int kWideSeqs = 384;  // the smallest batch of this kernel
 constexpr int kWideQuads = 2, kWideThreads = (kWideQuads + 1) * kQuadWarps * 32;
